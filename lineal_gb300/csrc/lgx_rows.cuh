@@ -47,7 +47,7 @@ struct RowCfg {
 };
 // upper bound of the CTAs per SM of every row-engine configuration:
 // reduction partials of row kernels are sized sm_count() * kRowsMaxCtasPerSm
-constexpr int kRowsMaxCtasPerSm = 16;
+constexpr int kRowsMaxCtasPerSm = 20;
 
 // per stage: row offsets (kTileRows + 4) * 8 bytes, columns (CAP + 8) * 4
 // bytes, values (CAP + 8) * sizeof(VT) bytes (an aligned span exceeds its
@@ -149,10 +149,10 @@ __device__ __forceinline__ void issue_tile(const int64_t *rowptr, const int32_t 
 
 // Op interface:
 //   using X = <type of the gathered vector entries>;
-//   template <int W> __device__ double row(int64_t row, const int32_t *c, const VT *v,
-//                                          int len) const;
+//   template <int W, bool FLAT> __device__ double row(int64_t row, const int32_t *c,
+//                                                     const VT *v, int len) const;
 //     (returns the row's contribution to an optional sum; W = entries whose
-//     gathers are issued together)
+//     gathers are issued together; FLAT: products without branches, row_dot)
 //   static constexpr bool kReduce;  __device__ void finish(double total) const;
 //   double *partials; unsigned *counter;  (when kReduce)
 template <typename VT, class Op, int KIND>
@@ -236,12 +236,12 @@ __global__ void __launch_bounds__(kTileRows, RowCfg<VT, KIND>::ctas_per_sm)
       if (row < cur.r1) {
         const Stage<VT> sg = stage(s);
         const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
-        contrib += op.template row<RowCfg<VT, KIND>::gather>(row, sg.col + (b - c0), sg.val + (b - v0),
+        contrib += op.template row<RowCfg<VT, KIND>::gather, false>(row, sg.col + (b - c0), sg.val + (b - v0),
                                                              (int)(e - b));
       }
     } else if (row < cur.r1) {
       const int64_t b = rowptr[row], e = rowptr[row + 1];
-      contrib += op.template row<RowCfg<VT, KIND>::gather>(row, col + b, val + b, (int)(e - b));
+      contrib += op.template row<RowCfg<VT, KIND>::gather, false>(row, col + b, val + b, (int)(e - b));
     }
     __syncthreads();
     if (NST == 1 && threadIdx.x == 0 && t + G < ntiles) {
@@ -306,6 +306,12 @@ __host__ __device__ constexpr size_t wsmem_bytes(int wpc, int nst, int capw, siz
   return wheader_bytes(wpc, nst) + (size_t)wpc * nst * wstage_bytes(capw, vsize);
 }
 
+// one-warp CTAs per SM that the registers of rows in rounds of 32, 16 and 8
+// gathers are capped for
+constexpr int kSmallMb32 = 10, kSmallMb16 = 14, kSmallMb8 = 20;
+// four-warp CTAs per SM of products whose rows have at most 8 entries
+constexpr int kShortMb = 6;
+
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -319,9 +325,14 @@ struct WrowsBounds {
   // within them; 8 warps per CTA: two CTAs (16 warps), 16 gathers per round;
   // MB = 7 (4 warps): seven CTAs (28 warps) where shared memory allows it
   // (float and bfloat16 stages), 16 float (8 double) gathers per round
-  // within 73 registers
+  // within 73 registers; one warp per CTA (launches of few tiles, see
+  // launch_small): 8, 16 or 32 gathers per round
   static constexpr int min_blocks = MB ? MB : (WPC == 4 ? 5 : 2);
-  static constexpr int gather = (WPC == 4 && sizeof(XT) == 8) ? 8 : 16;
+  static constexpr int gather = WPC == 1   ? (MB == kSmallMb32 ? 32 : MB == kSmallMb16 ? 16 : 8)
+                                : (WPC == 4 && sizeof(XT) == 8) ? 8
+                                                                : 16;
+  // products of rows without branches (row_dot)
+  static constexpr bool flat = WPC == 1 || MB == kShortMb;
 };
 
 template <typename VT, class Op, int WPC, int S, int MB = 0>
@@ -407,11 +418,11 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
       const int64_t c0 = e0 & ~(CA - 1), v0 = e0 & ~(VA - 1);
       if (row < r1) {
         const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
-        contrib += op.template row<W>(row, sg.col + (b - c0), sg.val + (b - v0), (int)(e - b));
+        contrib += op.template row<W, WrowsBounds<WPC, typename Op::X, MB>::flat>(row, sg.col + (b - c0), sg.val + (b - v0), (int)(e - b));
       }
     } else if (row < r1) {
       const int64_t b = rowptr[row], e = rowptr[row + 1];
-      contrib += op.template row<W>(row, col + b, val + b, (int)(e - b));
+      contrib += op.template row<W, WrowsBounds<WPC, typename Op::X, MB>::flat>(row, col + b, val + b, (int)(e - b));
     }
     __syncwarp();
     if (lane == 0 && t + S * GW < ntiles) {
@@ -445,6 +456,21 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
 // for seven CTAs per SM
 int rows_config();
 
+// Whether a row launch carries the programmatic-dependent-launch attribute.
+// Float rows do; FP64 rows up to pdl_fp64_rows(), except launches of long
+// rows (over 16 entries on average) in more tiles than SMs: their warps fill
+// the FP64 pipe, and an early-scheduled successor takes the SMs that the
+// running launch left free, so that its own warps pile up there.  27-point
+// colour launches, FP64, with / without: 3.7k rows 4.1 / 4.7 us, 6.9k 5.5 /
+// 4.8, 10.8k 6.1 / 5.1, 16k 6.5 / 6.1; 7-point 5.5k rows 2.4 / 3.3 us, 18k
+// 3.2 / 3.5, 167k 9.8 / 10.8.
+template <typename XT>
+inline bool rows_pdl(int64_t rb, int64_t re, const Csr &a) {
+  if (sizeof(XT) == 4) return true;
+  return re - rb <= pdl_fp64_rows() &&
+         (a.nnz <= 16 * a.n || re - rb <= (int64_t)sm_count() * kWarpTileRows);
+}
+
 template <typename VT, class Op, int WPC, int S, int MB = 0>
 inline lgx_status launch_wrows(int64_t rb, int64_t re, const Csr &a, const VT *val, const Op &op,
                                cudaStream_t s, bool *done) {
@@ -476,7 +502,7 @@ inline lgx_status launch_wrows(int64_t rb, int64_t re, const Csr &a, const VT *v
   const int64_t need = (tiles + WPC - 1) / WPC;
   const int64_t g = (int64_t)sm_count() * per_sm;
   const unsigned grid = (unsigned)(need < g ? (need > 0 ? need : 1) : g);
-  const bool pdl = sizeof(typename Op::X) == 4 || re - rb <= pdl_fp64_rows();
+  const bool pdl = rows_pdl<typename Op::X>(rb, re, a);
   LGX_CUDA(launch_pdl(pdl, k_wrows<VT, Op, WPC, S, MB>, dim3(grid),
                       dim3(WPC * 32), smem, s, rb, re, capw,
                       (const int64_t *)a.rowptr.p, (const int32_t *)a.col.p, val, op,
@@ -518,6 +544,25 @@ struct TuneClass<Op, std::void_t<decltype(Op::kTuneClass)>> {
   static constexpr int value = Op::kTuneClass;
 };
 
+// Launches of few tiles (the colours of small levels) in one-warp CTAs: the
+// warps spread evenly over the SMs, and with the rows' whole length in one or
+// two rounds of gathers the launch is one gather latency long.  Up to eight
+// tiles per SM, where the launch is latency-bound; beyond, four-warp CTAs
+// with shorter rounds keep more rows resident.  Colour launches, four-warp /
+// one-warp CTAs: 27-point FP64 3.7k rows 5.1 / 4.1 us, 16k 9.3 / 6.5, 28k
+// 10.7 / 9.6 (float 3.3 / 2.8, 4.3 / 3.7, 4.9 / 4.3), 55k 12.0 / 12.6 (float
+// 5.3 / 5.6); 7-point float 5.5k rows 2.0 / 1.8 us, 37k 2.4 / 2.2, 167k 5.2 /
+// 5.2.
+template <typename VT, class Op>
+inline lgx_status launch_small(int64_t rb, int64_t re, const Csr &a, const VT *val, const Op &op,
+                               cudaStream_t s, bool *done) {
+  if (re - rb > (int64_t)sm_count() * 8 * kWarpTileRows) return LGX_OK;
+  if (a.max_row <= 8) return launch_wrows<VT, Op, 1, 1, kSmallMb8>(rb, re, a, val, op, s, done);
+  if (a.max_row <= 16)
+    return launch_wrows<VT, Op, 1, 1, kSmallMb16>(rb, re, a, val, op, s, done);
+  return launch_wrows<VT, Op, 1, 1, kSmallMb32>(rb, re, a, val, op, s, done);
+}
+
 // rows [rb, re) of `a` (values `val`) through the engine configuration the
 // autotuner chose for this matrix and operation, else the process-wide one
 template <typename VT, class Op>
@@ -527,6 +572,16 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
   bool done = false;
   const int tuned = a.tuned[TuneClass<Op>::value][tune_value_index<VT>()];
   const int cfg = tuned >= 0 ? tuned : rows_config();
+  if constexpr (!Op::kReduce) {  // (a reduction wants few, large CTAs)
+    if (cfg == 3 || cfg == 7) LGX_CHECK((launch_small<VT, Op>(rb, re, a, val, op, s, &done)));
+    if (done) return LGX_OK;
+  }
+  // rows of at most 8 entries (7-point operators) at 256^3: FP64 product 350
+  // -> 274, float 295 -> 245 us
+  if (TuneClass<Op>::value == 0 && cfg == 3 && a.max_row <= 8) {
+    LGX_CHECK((launch_wrows<VT, Op, 4, 1, kShortMb>(rb, re, a, val, op, s, &done)));
+    if (done) return LGX_OK;
+  }
   switch (cfg) {
     case 3: LGX_CHECK((launch_wrows<VT, Op, 4, 1>(rb, re, a, val, op, s, &done))); break;
     case 4: LGX_CHECK((launch_wrows<VT, Op, 4, 2>(rb, re, a, val, op, s, &done))); break;
@@ -547,18 +602,59 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
 }
 
 // ---- row operations ---------------------------------------------------------
-// sum_k fma(a_k, x[c_k], init) in storage order.  The column and x loads of
-// up to W entries are issued together ahead of the dependent FMA chain, so a
-// 27-point row costs one (W = 32) or two (W = 16) rounds of gather latency.
-template <int W, typename VT, typename XT>
+// A row runs in chunks of W entries: the chunk's columns leave the stage
+// together, then all its x gathers go out, then the dependent FMA chain runs.
+// Nothing in the first two steps branches (entries past the row's end repeat
+// its last column index and load nothing), so a chunk costs one shared-memory
+// and one gather latency however long it is.  Written as a branch per entry,
+// each entry paid its own shared-memory latency twice (~110 cycles an entry:
+// 27-point colour launches of 2k rows, FP64 5.2, float 3.4 us).
+template <typename T>
+__device__ __forceinline__ void ld_if(T &v, const T *p, bool on);
+template <>
+__device__ __forceinline__ void ld_if<double>(double &v, const double *p, bool on) {
+  asm volatile(
+    "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+    "@p ld.global.f64 %0, [%1];\n\t}"
+    : "=d"(v)
+    : "l"(p), "r"((int)on));
+}
+template <>
+__device__ __forceinline__ void ld_if<float>(float &v, const float *p, bool on) {
+  asm volatile(
+    "{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+    "@p ld.global.f32 %0, [%1];\n\t}"
+    : "=f"(v)
+    : "l"(p), "r"((int)on));
+}
+
+// columns of entries k .. k + W - 1 (the last entry's past the row's end)
+template <int W>
+__device__ __forceinline__ void row_columns(const int32_t *c, int k, int len, int32_t (&cc)[W]) {
+#pragma unroll
+  for (int u = 0; u < W; ++u) cc[u] = c[min(k + u, len - 1)];
+}
+
+// sum_k fma(a_k, x[c_k], init) in storage order; FLAT: chunks as above, else
+// a branch per entry (what long rows in long launches want: bound by
+// bandwidth, they lose to the added tests -- 27 points at 200 x 181 x 150,
+// FP64: 323 us against 354)
+template <int W, bool FLAT, typename VT, typename XT>
 __device__ __forceinline__ XT row_dot(const int32_t *c, const VT *v, int len,
                                       const XT *__restrict__ x, XT sum) {
   for (int k = 0; k < len; k += W) {
     const int m = len - k < W ? len - k : W;
     XT xv[W];
+    if constexpr (FLAT) {
+      int32_t cc[W];
+      row_columns<W>(c, k, len, cc);
 #pragma unroll
-    for (int u = 0; u < W; ++u)
-      if (u < m) xv[u] = __ldg(x + c[k + u]);
+      for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], u < m);
+    } else {
+#pragma unroll
+      for (int u = 0; u < W; ++u)
+        if (u < m) xv[u] = __ldg(x + c[k + u]);
+    }
 #pragma unroll
     for (int u = 0; u < W; ++u)
       if (u < m) sum = fma(cvt<XT>(v[k + u]), xv[u], sum);

@@ -31,7 +31,7 @@ struct JacobiOp {
   static constexpr bool kReduce = false;
   double *partials = nullptr;
   unsigned *counter = nullptr;
-  template <int W>
+  template <int W, bool FLAT>
   __device__ __forceinline__ double row(int64_t i, const int32_t *c, const VT *v, int len) const {
     double accum = b[i], diag = 0.0;
     for (int k = 0; k < len; ++k) {
@@ -391,24 +391,28 @@ struct SorOp {
   static constexpr int kTuneClass = 1;
   double *partials = nullptr;
   unsigned *counter = nullptr;
-  template <int W>
+  template <int W, bool FLAT>
   __device__ __forceinline__ double row(int64_t i, const int32_t *c, const VT *v, int len) const {
     if constexpr (kIsBf16<VT>) {
       return row_scaled<W>(i, c, v, len);
     }
     XT accum = b[i], diag = XT(0);
     const XT xi = from_zero ? XT(0) : x[i];
+    const int64_t end = from_zero ? visit_end : INT64_MAX;
+    // constant, so it loads with the row's first loads
+    const double y = sizeof(XT) == 8 && rdiag ? rdiag[i] : 0.0;
     for (int k = 0; k < len; k += W) {
-      const int m = len - k < W ? len - k : W;
+      const int m = len - k;
+      int32_t cc[W];
       XT xv[W];
+      row_columns<W>(c, k, len, cc);
 #pragma unroll
-      for (int u = 0; u < W; ++u)
-        if (u < m) xv[u] = (from_zero && c[k + u] >= visit_end) ? XT(0) : x[c[k + u]];
+      for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], u < m && cc[u] != i && cc[u] < end);
 #pragma unroll
       for (int u = 0; u < W; ++u) {
         if (u < m) {
           const XT a = cvt<XT>(v[k + u]);
-          if (c[k + u] == i) {
+          if (cc[u] == i) {
             diag = a;
             if (ultra) accum = fma(-a, xi, accum);
           } else {
@@ -423,7 +427,6 @@ struct SorOp {
     }
     XT quot;
     if constexpr (sizeof(XT) == 8) {
-      const double y = rdiag ? rdiag[i] : 0.0;
       quot = (nonzero_bits(y) && exponent_within_400(accum)) ? div_by_recip(accum, diag, y)
                                                              : accum / diag;
       if (relax_one && nonzero_bits(quot) && exponent_field(xi) != 0x7ff) {
@@ -445,17 +448,19 @@ struct SorOp {
     const XT si = scale[i];
     const XT xi = from_zero ? XT(0) : x[i];
     XT t = XT(0), vd = XT(0);
+    const int64_t end = from_zero ? visit_end : INT64_MAX;
     for (int k = 0; k < len; k += W) {
-      const int m = len - k < W ? len - k : W;
+      const int m = len - k;
+      int32_t cc[W];
       XT xv[W];
+      row_columns<W>(c, k, len, cc);
 #pragma unroll
-      for (int u = 0; u < W; ++u)
-        if (u < m) xv[u] = (from_zero && c[k + u] >= visit_end) ? XT(0) : x[c[k + u]];
+      for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], u < m && cc[u] != i && cc[u] < end);
 #pragma unroll
       for (int u = 0; u < W; ++u) {
         if (u < m) {
           const XT a = cvt<XT>(v[k + u]);
-          if (c[k + u] == i) {
+          if (cc[u] == i) {
             vd = a;
           } else {
             t = fma(a, xv[u], t);

@@ -31,9 +31,9 @@ struct SpmvOp {
   static constexpr bool kReduce = false;
   double *partials = nullptr;
   unsigned *counter = nullptr;
-  template <int W>
+  template <int W, bool FLAT>
   __device__ __forceinline__ double row(int64_t i, const int32_t *c, const VT *v, int len) const {
-    y[i] = row_dot<W, VT, XT>(c, v, len, x, XT(0));
+    y[i] = row_dot<W, FLAT, VT, XT>(c, v, len, x, XT(0));
     return 0.0;
   }
   __device__ __forceinline__ void finish(double) const {}
@@ -50,9 +50,9 @@ struct ResidualOp {
   double *partials;
   unsigned *counter;
   const float *scale = nullptr;  // bfloat16 values: row factor
-  template <int W>
+  template <int W, bool FLAT>
   __device__ __forceinline__ double row(int64_t i, const int32_t *c, const VT *v, int len) const {
-    XT ax = row_dot<W, VT, XT>(c, v, len, x, XT(0));
+    XT ax = row_dot<W, FLAT, VT, XT>(c, v, len, x, XT(0));
     if constexpr (kIsBf16<VT>) ax = ax * scale[i];
     const XT rv = b[i] - ax;
     r[i] = rv;
