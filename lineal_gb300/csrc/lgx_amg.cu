@@ -2573,6 +2573,18 @@ static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
       continue;
     }
     lv.col = std::make_unique<lgx_colouring>();
+    // Levels with a colouring of their own keep their vectors in natural
+    // order: a warp's rows then gather from a few lines of x (32 rows of one
+    // of c colours span 32 c consecutive x), where in colour order each of
+    // their gathers sits in another colour's block, in a line of its own, and
+    // the L1's one line per cycle bounds a colour's launch.  With the rows'
+    // halves (a sweep from zero and the residual after it read half the
+    // matrix each): float-vector AMG-CG at 256^3, 7 points, 348 -> 290 ms, at
+    // 121 x 117 x 125, 27 points, 73 -> 67; FP64 at 256^3, 27 points, 535 ->
+    // 501.  A given finest
+    // colouring keeps colour order, which is the order its grid kernels need;
+    // bfloat16 values keep it too.
+    const bool natural = !(l == 0 && finest_colouring) && !(h.f32 && p.cycle_bf16);
     if (l == 0 && finest_colouring) {
       LGX_CHECK(colouring_build(*lv.a, finest_colouring->colour.p, finest_colouring->ncolours, s,
                                 *lv.col));
@@ -2582,7 +2594,23 @@ static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
         LGX_CHECK(colouring_smallest_last(*lv.a, s, lv.col->colour, nc));
       else
         LGX_CHECK(colouring_jp(*lv.a, p.colour_seed + (uint64_t)l, s, lv.col->colour, nc));
-      LGX_CHECK(colouring_build(*lv.a, lv.col->colour.p, nc, s, *lv.col));
+      if (natural)
+        LGX_CHECK(colouring_build_natural(*lv.a, lv.col->colour.p, nc, h.f32, s, *lv.col));
+      else
+        LGX_CHECK(colouring_build(*lv.a, lv.col->colour.p, nc, s, *lv.col));
+    }
+    if (natural) {
+      if (l == 0 && h.f32 && lv.a->storage == LGX_F64) {
+        const int64_t nnz = lv.a->nnz;
+        LGX_CHECK(lv.nat32.alloc(nnz + kCsrPad));
+        if (nnz) {
+          k_convert<double, float><<<std::min<int64_t>(grid_for(nnz, 256), 16384), 256, 0, s>>>(
+            nnz, lv.a->v64.p, lv.nat32.p);
+          LGX_LAUNCH_CHECK();
+        }
+      }
+      timer.mark(s, "colouring", l);
+      continue;
     }
     if (h.f32) LGX_CHECK(colouring_make_f32(*lv.col, s));
     if (h.f32 && p.cycle_bf16) LGX_CHECK(colouring_make_bf16(*lv.col, s));
@@ -2596,12 +2624,12 @@ static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
   for (int64_t l = 0; l + 1 < L; ++l) {
     lgx_amg_level &f = *h.lv[l];
     lgx_amg_level &c = *h.lv[l + 1];
-    const int32_t *perm_c = c.col ? c.col->perm.p : nullptr;
-    const int32_t *iperm_c = c.col ? c.col->iperm.p : nullptr;
+    const int32_t *perm_c = c.perm();
+    const int32_t *iperm_c = c.iperm();
     const int64_t nf = f.a->n, nc = c.a->n;
     LGX_CHECK(f.agg_p.alloc(nf));
     k_agg_permute<<<std::min<int64_t>(grid_for(nf, 256), 16384), 256, 0, s>>>(
-      nf, f.col->perm.p, f.agg.agg.p, iperm_c, f.agg_p.p);
+      nf, f.perm(), f.agg.agg.p, iperm_c, f.agg_p.p);
     LGX_LAUNCH_CHECK();
     DBuf<int64_t> len;
     LGX_CHECK(len.alloc(nc));
@@ -2616,7 +2644,7 @@ static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
     LGX_CHECK(f.rlist.alloc(total));
     if (nc) {
       k_rlist_fill<<<std::min<int64_t>(grid_for(nc, 256), 16384), 256, 0, s>>>(
-        nc, perm_c, f.agg.list_ptr.p, f.agg.list.p, f.col->iperm.p, f.rptr.p, f.rlist.p);
+        nc, perm_c, f.agg.list_ptr.p, f.agg.list.p, f.iperm(), f.rptr.p, f.rlist.p);
       LGX_LAUNCH_CHECK();
     }
     LGX_CUDA(cudaStreamSynchronize(s));
@@ -2707,6 +2735,16 @@ static lgx_status level_residual(lgx_amg_level &lv, const lgx_amg &h, const XT *
       return matrix_residual(lv.stencil, b, x, r, nullptr, nullptr, nullptr, s);
     else
       return fail(LGX_ERR_UNSUPPORTED, "a stencil finest level runs the FP64 cycle");
+  }
+  if (c.natural) {
+    // every residual of the cycle follows a forward sweep from zero
+    const bool up = h.p.smoother_relax == 1.0 && !h.p.smoother_ultra;
+    if constexpr (sizeof(XT) == 8)
+      if (c.pcsr.storage == LGX_F64)
+        return up ? mc_up_residual<double, double>(c, x, r, s)
+                  : mc_residual<double, double>(c, c.pcsr.v64.p, b, x, r, s);
+    return up ? mc_up_residual<float, XT>(c, x, r, s)
+              : mc_residual<float, XT>(c, c.pcsr.v32.p, b, x, r, s);
   }
   if constexpr (sizeof(XT) == 8) {
     if (c.pcsr.storage == LGX_F64)
@@ -2825,8 +2863,8 @@ static lgx_status vcycle_impl(lgx_amg &h, const XT *b0, XT *x0, cudaStream_t s) 
   return LGX_OK;
 }
 
-const Csr &amg_finest_permuted(const lgx_amg &h) { return h.lv[0]->col->pcsr; }
 lgx_colouring *amg_finest_colouring(lgx_amg &h) { return h.lv[0]->col.get(); }
+const Csr &amg_finest_matrix(const lgx_amg &h) { return *h.lv[0]->a; }
 
 // Applies the preconditioner in the finest level's permuted space with
 // double vectors (the outer Krylov vectors).
@@ -2853,9 +2891,11 @@ lgx_status amg_apply_permuted_f32(lgx_amg &h, const float *b, float *x, cudaStre
   if (!h.f32) return fail(LGX_ERR_UNSUPPORTED, "float V-cycle needs a cycle_f32 hierarchy");
   return vcycle_impl<float>(h, b, x, s);
 }
-// float values of the finest permuted matrix (the cycle's own copy)
+// float values of the finest matrix in the cycle's order (natural or permuted)
 const float *amg_finest_values_f32(const lgx_amg &h) {
-  const lgx_colouring &c = *h.lv[0]->col;
+  const lgx_amg_level &l0 = *h.lv[0];
+  const lgx_colouring &c = *l0.col;
+  if (c.natural) return l0.a->storage == LGX_F32 ? l0.a->v32.p : l0.nat32.p;
   return c.pcsr.storage == LGX_F32 ? c.pcsr.v32.p : c.pv32.p;
 }
 
@@ -3163,7 +3203,7 @@ lgx_status lgx_amg_vcycle(lgx_amg *h, const double *d_b, double *d_x, lgx_stream
     LGX_CHECK(h->nat_b.alloc(n));
     LGX_CHECK(h->nat_x.alloc(n));
   }
-  const int32_t *perm = h->lv.size() > 1 ? l0.col->perm.p : nullptr;
+  const int32_t *perm = h->lv.size() > 1 ? l0.perm() : nullptr;
   if (perm) {
     LGX_CHECK(gather<double, double>(n, perm, d_b, h->nat_b.p, stream));
     LGX_CHECK(amg_apply_permuted(*h, h->nat_b.p, h->nat_x.p, stream));

@@ -28,12 +28,18 @@ struct lgx_amg_level {
   lgx::DBuf<uint32_t> agg_p;         // permuted fine -> permuted coarse
   lgx::DBuf<int64_t> rptr;           // permuted coarse row -> fine rows (permuted)
   lgx::DBuf<int32_t> rlist;
-  lgx::DBuf<double> b64, x64, r64;   // cycle vectors (permuted order)
+  lgx::DBuf<double> b64, x64, r64;   // cycle vectors (in the level's order, see perm())
   lgx::DBuf<float> b32, x32, r32;
   // level 0 of a hierarchy built on a stencil matrix: the smoother and the
   // residual run matrix-free on it (red-black, natural order); `own` then
   // keeps only the sizes of the assembled matrix the setup used
   const lgx_matrix *stencil = nullptr;
+  // float values of `a` in natural order (level 0 of a natural-order float
+  // cycle: the products of the float-vector CG)
+  lgx::DBuf<float> nat32;
+  // colour order -> natural order of the level's vectors; null: natural order
+  const int32_t *perm() const { return col && !col->natural ? col->perm.p : nullptr; }
+  const int32_t *iperm() const { return col && !col->natural ? col->iperm.p : nullptr; }
 };
 
 struct lgx_amg {
@@ -46,5 +52,6 @@ struct lgx_amg {
   int32_t stop_reason = 0;           // LGX_STOP_* (hierarchy/wright.hpp:26-28)
   lgx::DBuf<double> nat_b, nat_x;    // natural-order staging for lgx_amg_vcycle
   bool f32 = false;
+  bool tuned_outer = false;          // the autotuner set the finest matrix's product slot
 };
 

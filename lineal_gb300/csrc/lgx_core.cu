@@ -202,44 +202,56 @@ lgx_status csr_compute_max_row(Csr &a, cudaStream_t s) {
   return LGX_OK;
 }
 
-// the block's maximum first, one atomic per block (one per row on a single
+// the most entries in any kWarpTileRows consecutive rows and in any row; the
+// block's maximum first, one atomic per block (one per row on a single
 // address serialised 16.8M atomics at 256^3: 8 ms)
-__global__ void __launch_bounds__(256) k_csr_window(int64_t n, const int64_t *rowptr,
-                                                    unsigned long long *max_win) {
-  __shared__ unsigned long long part[8];
-  unsigned long long m = 0;
+__global__ void __launch_bounds__(256) k_csr_extents(int64_t n, const int64_t *rowptr,
+                                                     unsigned long long *mx) {
+  __shared__ unsigned long long part[2][8];
+  unsigned long long m[2] = {0, 0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = rowptr[i];
+    const int64_t b = rowptr[i], e = rowptr[i + 1];
     const int64_t we = rowptr[i + kWarpTileRows < n ? i + kWarpTileRows : n];
-    m = (unsigned long long)(we - b) > m ? (unsigned long long)(we - b) : m;
+    m[0] = max(m[0], (unsigned long long)(we - b));
+    m[1] = max(m[1], (unsigned long long)(e - b));
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
-    m = q > m ? q : m;
-  }
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+  for (int o = 16; o > 0; o >>= 1)
+    for (int q = 0; q < 2; ++q) m[q] = max(m[q], __shfl_xor_sync(0xffffffffu, m[q], o));
+  if ((threadIdx.x & 31) == 0)
+    for (int q = 0; q < 2; ++q) part[q][threadIdx.x >> 5] = m[q];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = part[w] > m ? part[w] : m;
-    atomicMax(max_win, m);
+  if (threadIdx.x < 2) {
+    unsigned long long v = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v = max(v, part[threadIdx.x][w]);
+    atomicMax(&mx[threadIdx.x], v);
   }
 }
 
-lgx_status csr_compute_max_window(Csr &a, cudaStream_t s) {
+lgx_status csr_compute_extents(Csr *const *list, int count, cudaStream_t s) {
   DBuf<unsigned long long> mx;
-  LGX_CHECK(mx.alloc(1));
-  LGX_CUDA(cudaMemsetAsync(mx.p, 0, sizeof(unsigned long long), s));
-  if (a.n) {
-    k_csr_window<<<std::min<int64_t>(grid_for(a.n, 256), 4096), 256, 0, s>>>(a.n, a.rowptr.p,
-                                                                              mx.p);
+  LGX_CHECK(mx.alloc(2 * count));
+  LGX_CUDA(cudaMemsetAsync(mx.p, 0, 2 * count * sizeof(unsigned long long), s));
+  for (int k = 0; k < count; ++k) {
+    const Csr &a = *list[k];
+    if (a.n == 0) continue;
+    k_csr_extents<<<std::min<int64_t>(grid_for(a.n, 256), 4096), 256, 0, s>>>(a.n, a.rowptr.p,
+                                                                               mx.p + 2 * k);
     LGX_LAUNCH_CHECK();
   }
-  unsigned long long h = 0;
-  LGX_CUDA(cudaMemcpyAsync(&h, mx.p, sizeof(h), cudaMemcpyDeviceToHost, s));
+  std::vector<unsigned long long> h(2 * (size_t)count, 0);
+  LGX_CUDA(cudaMemcpyAsync(h.data(), mx.p, h.size() * sizeof(h[0]), cudaMemcpyDeviceToHost, s));
   LGX_CUDA(cudaStreamSynchronize(s));
-  a.max_win = (int64_t)h;
+  for (int k = 0; k < count; ++k) {
+    list[k]->max_win = (int64_t)h[2 * k];
+    list[k]->max_row = (int64_t)h[2 * k + 1];
+  }
   return LGX_OK;
+}
+
+lgx_status csr_compute_max_window(Csr &a, cudaStream_t s) {
+  Csr *one[1] = {&a};
+  return csr_compute_extents(one, 1, s);
 }
 
 // ---------------------------------------------------------------------------

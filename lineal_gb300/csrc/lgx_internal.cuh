@@ -206,6 +206,15 @@ struct lgx_colouring {
   lgx::DBuf<double> work_b, work_x;  // natural<->permuted staging for the public sweep API
   bool stencil_rb = false;       // red-black colouring of a stencil matrix: the sweeps run
                                  // matrix-free in natural order (no permuted copy)
+  // A level whose vectors stay in natural order (AMG levels without a given
+  // finest colouring): pcsr keeps its rows in colour order, row r being row
+  // perm[r], but its columns are natural.
+  bool natural = false;
+  // Halves of such a level's rows, entries in row order: `lo` (rows in colour
+  // order) the entries in earlier colours, all that a forward sweep from zero
+  // reads; `up` (rows in natural order) those in later colours, all that the
+  // residual after such a sweep needs when relax is 1 (mc_up_residual).
+  lgx::Csr lo, up;
 };
 
 namespace lgx {
@@ -225,6 +234,8 @@ lgx_status csr_compute_max_row(Csr &a, cudaStream_t s);
 constexpr int kWarpTileRows = 32;
 // sets a.max_win from the row offsets (for matrices whose rows were permuted)
 lgx_status csr_compute_max_window(Csr &a, cudaStream_t s);
+// sets max_row and max_win of `count` matrices from their row offsets
+lgx_status csr_compute_extents(Csr *const *list, int count, cudaStream_t s);
 
 // y = A x for CSR with value type VT and vector type XT (accumulation in XT)
 template <typename VT, typename XT>
@@ -278,6 +289,10 @@ lgx_status dot(int64_t n, const double *a, const double *b, double *out, double 
 // colouring helpers
 lgx_status colouring_build(const Csr &a, const int32_t *d_colour, int32_t ncolours,
                            cudaStream_t s, lgx_colouring &out);
+// the natural-order form (lgx_colouring::natural) with its halves; f32: values
+// stored as float
+lgx_status colouring_build_natural(const Csr &a, const int32_t *d_colour, int32_t ncolours,
+                                   bool f32, cudaStream_t s, lgx_colouring &out);
 lgx_status colouring_jp(const Csr &a, uint64_t seed, cudaStream_t s, DBuf<int32_t> &colour,
                         int32_t &ncolours);
 // One multicolour sweep on the permuted matrix (vectors in permuted order,
@@ -294,6 +309,15 @@ lgx_status mc_sor_sweep(const lgx_colouring &c, const VT *val, double relax, int
                         const float *scale = nullptr, XT *r_last = nullptr,
                         int64_t *res_from = nullptr);
 lgx_status colouring_make_bf16(lgx_colouring &c, cudaStream_t s);
+// b - A x of a natural-order level
+template <typename VT, typename XT>
+lgx_status mc_residual(const lgx_colouring &c, const VT *val, const XT *b, const XT *x, XT *r,
+                       cudaStream_t s);
+// The residual of a natural-order level right after a forward sweep from zero
+// with relax 1 (not ultra): the sweep solved every row with its earlier
+// colours, (D + L) x = b, so what is left is -U x.
+template <typename VT, typename XT>
+lgx_status mc_up_residual(const lgx_colouring &c, const XT *x, XT *r, cudaStream_t s);
 // gives c.pcsr a Grid27 when it is the parity-coloured 27-point (points 27)
 // or red-black 7-point (points 7) operator on `dims` (checked on the device;
 // *attached tells whether it was)

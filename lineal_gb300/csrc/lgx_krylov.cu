@@ -19,8 +19,8 @@
 
 namespace lgx {
 lgx_status amg_apply_permuted(lgx_amg &h, const double *b, double *x, cudaStream_t s);
-const Csr &amg_finest_permuted(const lgx_amg &h);
 lgx_colouring *amg_finest_colouring(lgx_amg &h);
+const Csr &amg_finest_matrix(const lgx_amg &h);
 bool amg_cycle_f32(const lgx_amg &h);
 lgx_status amg_apply_permuted_f32(lgx_amg &h, const float *b, float *x, cudaStream_t s);
 const float *amg_finest_values_f32(const lgx_amg &h);
@@ -218,8 +218,8 @@ __global__ void k_bicg_init(KScalars *ks) {
 // ---------------------------------------------------------------------------
 struct Solver {
   const lgx_matrix *m = nullptr;  // natural-order operator (when pcsr == nullptr)
-  const Csr *pcsr = nullptr;      // permuted CSR operator
-  const int32_t *perm = nullptr;  // permuted -> natural (when pcsr)
+  const Csr *pcsr = nullptr;      // CSR operator in the preconditioner's order
+  const int32_t *perm = nullptr;  // that order -> natural; null: natural order
   int precon = LGX_PRECON_NONE;
   double relax = 1.0;
   int ultra = 0;
@@ -241,6 +241,17 @@ struct Solver {
     LGX_CHECK(ks.alloc(1));
     LGX_CUDA(cudaMemsetAsync(counters.p, 0, 2 * sizeof(unsigned), s));
     LGX_CUDA(cudaMemsetAsync(ks.p, 0, sizeof(KScalars), s));
+    return LGX_OK;
+  }
+  // vectors between the caller's (natural) order and the solver's
+  lgx_status load(const double *src, double *dst) {
+    if (perm) return gather<double, double>(n, perm, src, dst, s);
+    LGX_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+    return LGX_OK;
+  }
+  lgx_status store(const double *src, double *dst) {
+    if (perm) return scatter<double, double>(n, perm, src, dst, s);
+    LGX_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     return LGX_OK;
   }
   lgx_status apply(const double *x, double *y) {
@@ -345,6 +356,8 @@ static lgx_status setup_solver(const lgx_matrix *a, const lgx_solve_params *p, c
           // the stencil itself
           if (a->kind == LGX_MATRIX_CSR)
             return fail(LGX_ERR_INVALID, "the hierarchy was built on a stencil matrix");
+        } else if (c->natural) {
+          S.pcsr = &amg_finest_matrix(*p->amg);  // natural order: the matrix as it is
         } else {
           S.pcsr = &c->pcsr;
           S.perm = c->perm.p;
@@ -411,13 +424,8 @@ static lgx_status krylov_init(lgx_krylov &K, const double *d_b, const double *d_
   LGX_CHECK(K.V.alloc(cg ? (flexible ? 6 : 5) : 8, n));
   double *b = K.V[0], *x = K.V[1], *r = K.V[2];
   cudaStream_t s = S.s;
-  if (S.perm) {
-    LGX_CHECK(gather<double, double>(n, S.perm, d_b, b, s));
-    LGX_CHECK(gather<double, double>(n, S.perm, d_x, x, s));
-  } else {
-    LGX_CUDA(cudaMemcpyAsync(b, d_b, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    LGX_CUDA(cudaMemcpyAsync(x, d_x, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  }
+  LGX_CHECK(S.load(d_b, b));
+  LGX_CHECK(S.load(d_x, x));
   KScalars *ks = S.ks.p;
   const unsigned rg = (unsigned)reduce_blocks(n);
   LGX_CHECK(S.residual(b, x, r, &ks->res2));
@@ -585,12 +593,7 @@ static lgx_status krylov_iterate(lgx_krylov &K) {
 }
 
 static lgx_status krylov_solution(lgx_krylov &K, double *d_x) {
-  const int64_t n = K.S.n;
-  if (K.S.perm) {
-    LGX_CHECK(scatter<double, double>(n, K.S.perm, K.V[1], d_x, K.S.s));
-  } else {
-    LGX_CUDA(cudaMemcpyAsync(d_x, K.V[1], sizeof(double) * n, cudaMemcpyDeviceToDevice, K.S.s));
-  }
+  LGX_CHECK(K.S.store(K.V[1], d_x));
   LGX_CUDA(cudaStreamSynchronize(K.S.s));
   return LGX_OK;
 }
@@ -922,8 +925,8 @@ static lgx_status run_refined(const lgx_matrix *a, const double *d_b, double *d_
   LGX_CHECK(R.x.alloc(n));
   LGX_CHECK(R.r.alloc(n));
   LGX_CHECK(R.alloc(n));
-  LGX_CHECK(gather<double, double>(n, S.perm, d_b, R.b.p, s));
-  LGX_CHECK(gather<double, double>(n, S.perm, d_x, R.x.p, s));
+  LGX_CHECK(S.load(d_b, R.b.p));
+  LGX_CHECK(S.load(d_x, R.x.p));
   KScalars *ks = S.ks.p;
   KScalars h{};
   const unsigned rg = (unsigned)reduce_blocks(n);
@@ -978,7 +981,7 @@ static lgx_status run_refined(const lgx_matrix *a, const double *d_b, double *d_
     // the refinement
     if (res >= prev) break;
   }
-  LGX_CHECK(scatter<double, double>(n, S.perm, R.x.p, d_x, s));
+  LGX_CHECK(S.store(R.x.p, d_x));
   LGX_CUDA(cudaStreamSynchronize(s));
   if (iterations) *iterations = it;
   if (final_rel) *final_rel = r0 > 0 ? res / r0 : 0.0;
@@ -1019,8 +1022,8 @@ static lgx_status run_reliable(const lgx_matrix *a, const double *d_b, double *d
   LGX_CHECK(R.r.alloc(n));
   R.flexible = p->flexible != 0;
   LGX_CHECK(R.alloc(n));
-  LGX_CHECK(gather<double, double>(n, S.perm, d_b, R.b.p, s));
-  LGX_CHECK(gather<double, double>(n, S.perm, d_x, R.x.p, s));
+  LGX_CHECK(S.load(d_b, R.b.p));
+  LGX_CHECK(S.load(d_x, R.x.p));
   KScalars *ks = S.ks.p;
   KScalars h{};
   const unsigned rg = (unsigned)reduce_blocks(n);
@@ -1085,7 +1088,7 @@ static lgx_status run_reliable(const lgx_matrix *a, const double *d_b, double *d
     res = std::sqrt(h.res2);
     if (history) history[it] = res;
   }
-  LGX_CHECK(scatter<double, double>(n, S.perm, R.x.p, d_x, s));
+  LGX_CHECK(S.store(R.x.p, d_x));
   LGX_CUDA(cudaStreamSynchronize(s));
   if (iterations) *iterations = it;
   if (final_rel) *final_rel = r0 > 0 ? res / r0 : 0.0;

@@ -37,15 +37,19 @@ inline unsigned mgrid(int64_t rows) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(g, 65535));
 }
 
-// y = A x (or r = b - A x with b != null) for rows [rb, re) of A, K columns
+// y = A x (r = b - A x with b != null, y = -A x with neg) for rows [rb, re) of
+// A, K columns; matrix row r is vector row rows[r] (natural-order levels), or
+// r itself
 template <typename VT, typename XT>
 __global__ void __launch_bounds__(kMThreads)
   k_mspmv(int64_t rb, int64_t re, const int64_t *__restrict__ rowptr,
-          const int32_t *__restrict__ col, const VT *__restrict__ val, int K,
-          const XT *__restrict__ b, const XT *__restrict__ x, XT *__restrict__ y) {
+          const int32_t *__restrict__ col, const VT *__restrict__ val,
+          const int32_t *__restrict__ rows, int K, int neg, const XT *__restrict__ b,
+          const XT *__restrict__ x, XT *__restrict__ y) {
   const int lane = threadIdx.x & 31;
-  for (int64_t i = rb + warp_id_global(); i < re; i += warps_global()) {
-    const int64_t e0 = rowptr[i], e1 = rowptr[i + 1];
+  for (int64_t r = rb + warp_id_global(); r < re; r += warps_global()) {
+    const int64_t e0 = rowptr[r], e1 = rowptr[r + 1];
+    const int64_t i = rows ? rows[r] : r;
     XT acc = XT(0);
     for (int64_t base = e0; base < e1; base += 32) {
       const int m = e1 - base < 32 ? (int)(e1 - base) : 32;
@@ -61,25 +65,29 @@ __global__ void __launch_bounds__(kMThreads)
         if (lane < K) acc = fma(a, x[(int64_t)c * K + lane], acc);
       }
     }
-    if (lane < K) y[i * K + lane] = b ? b[i * K + lane] - acc : acc;
+    if (lane < K) y[i * K + lane] = b ? b[i * K + lane] - acc : neg ? -acc : acc;
   }
 }
 
 // One colour of a multicolour SOR sweep on K columns (the row formula of
 // gauss-seidel-variant/sweep.hpp:134-200, in place).  from_zero: forward
-// sweep from x = 0, rows at or after visit_end read as 0.
+// sweep from x = 0, rows at or after visit_end read as 0.  With pdiag the rows
+// are a natural-order level's earlier-colour halves (all that such a sweep
+// reads) and their diagonals stand there.
 template <typename VT, typename XT>
 __global__ void __launch_bounds__(kMThreads)
   k_msor(int64_t rb, int64_t re, const int64_t *__restrict__ rowptr,
-         const int32_t *__restrict__ col, const VT *__restrict__ val, int K,
+         const int32_t *__restrict__ col, const VT *__restrict__ val,
+         const int32_t *__restrict__ rows, const double *__restrict__ pdiag, int K,
          const XT *__restrict__ b, XT *x, XT relax, XT m1, int ultra, int from_zero,
          int64_t visit_end) {
   const int lane = threadIdx.x & 31;
-  for (int64_t i = rb + warp_id_global(); i < re; i += warps_global()) {
-    const int64_t e0 = rowptr[i], e1 = rowptr[i + 1];
+  for (int64_t r = rb + warp_id_global(); r < re; r += warps_global()) {
+    const int64_t e0 = rowptr[r], e1 = rowptr[r + 1];
+    const int64_t i = rows ? rows[r] : r;
     XT accum = lane < K ? b[i * K + lane] : XT(0);
     const XT xi = (lane < K && !from_zero) ? x[i * K + lane] : XT(0);
-    XT diag = XT(0);
+    XT diag = pdiag ? (XT)pdiag[r] : XT(0);
     for (int64_t base = e0; base < e1; base += 32) {
       const int m = e1 - base < 32 ? (int)(e1 - base) : 32;
       int32_t c_l = 0;
@@ -241,52 +249,60 @@ struct MWork {
   std::vector<DBuf<XT>> b, x, r;
 };
 
-template <typename XT>
-static lgx_status m_level_sor(const lgx_amg &h, const lgx_amg_level &lv, int K, int forward,
-                              int from_zero, const XT *b, XT *x, cudaStream_t s) {
-  const lgx_colouring &c = *lv.col;
-  const Csr &p = c.pcsr;
-  const XT relax = (XT)h.p.smoother_relax, m1 = XT(1) - (XT)h.p.smoother_relax;
-  const int ultra = h.p.smoother_ultra;
+template <typename VT, typename XT>
+static lgx_status m_sor(const lgx_colouring &c, const VT *val, const VT *lo_val, int K, int forward,
+                        int from_zero, const XT *b, XT *x, XT relax, int ultra, cudaStream_t s) {
+  const int fz = from_zero && forward;
+  const bool halves = fz && c.natural;
+  const Csr &p = halves ? c.lo : c.pcsr;
+  const int32_t *rows = c.natural ? c.perm.p : nullptr;
   for (int32_t k = 0; k < c.ncolours; ++k) {
     const int32_t cid = forward ? k : c.ncolours - 1 - k;
     const int64_t rb = c.offsets[cid], re = c.offsets[cid + 1];
     if (re <= rb) continue;
-    const int fz = from_zero && forward;
-    if constexpr (sizeof(XT) == 8) {
-      if (p.storage == LGX_F64)
-        k_msor<double, double><<<mgrid(re - rb), kMThreads, 0, s>>>(
-          rb, re, p.rowptr.p, p.col.p, p.v64.p, K, b, x, relax, m1, ultra, fz, rb);
-      else
-        k_msor<float, double><<<mgrid(re - rb), kMThreads, 0, s>>>(
-          rb, re, p.rowptr.p, p.col.p, p.v32.p, K, b, x, relax, m1, ultra, fz, rb);
-    } else {
-      const float *v = p.storage == LGX_F32 ? p.v32.p : c.pv32.p;
-      k_msor<float, float><<<mgrid(re - rb), kMThreads, 0, s>>>(rb, re, p.rowptr.p, p.col.p, v,
-                                                                 K, b, x, relax, m1, ultra, fz,
-                                                                 rb);
-    }
+    k_msor<VT, XT><<<mgrid(re - rb), kMThreads, 0, s>>>(
+      rb, re, p.rowptr.p, p.col.p, halves ? lo_val : val, rows, halves ? c.pdiag.p : nullptr, K, b,
+      x, relax, XT(1) - relax, ultra, fz, halves ? INT64_MAX : rb);
     LGX_LAUNCH_CHECK();
   }
   return LGX_OK;
 }
 
 template <typename XT>
-static lgx_status m_level_residual(const lgx_amg_level &lv, int K, const XT *b, const XT *x,
-                                   XT *r, cudaStream_t s) {
-  const Csr &p = lv.col->pcsr;
+static lgx_status m_level_sor(const lgx_amg &h, const lgx_amg_level &lv, int K, int forward,
+                              int from_zero, const XT *b, XT *x, cudaStream_t s) {
+  const lgx_colouring &c = *lv.col;
+  const XT relax = (XT)h.p.smoother_relax;
+  const int ultra = h.p.smoother_ultra;
+  if constexpr (sizeof(XT) == 8)
+    if (c.pcsr.storage == LGX_F64)
+      return m_sor<double, XT>(c, c.pcsr.v64.p, c.lo.v64.p, K, forward, from_zero, b, x, relax,
+                               ultra, s);
+  const float *v = c.pcsr.storage == LGX_F32 ? c.pcsr.v32.p : c.pv32.p;
+  return m_sor<float, XT>(c, v, c.lo.v32.p, K, forward, from_zero, b, x, relax, ultra, s);
+}
+
+template <typename XT>
+static lgx_status m_level_residual(const lgx_amg &h, const lgx_amg_level &lv, int K, const XT *b,
+                                   const XT *x, XT *r, cudaStream_t s) {
+  const lgx_colouring &c = *lv.col;
+  // after a forward sweep from zero the later-colour halves are enough
+  // (mc_up_residual)
+  const bool up = c.natural && h.p.smoother_relax == 1.0 && !h.p.smoother_ultra;
+  const Csr &p = up ? c.up : c.pcsr;
+  const int32_t *rows = c.natural && !up ? c.perm.p : nullptr;
+  const XT *bb = up ? nullptr : b;
   if constexpr (sizeof(XT) == 8) {
-    if (p.storage == LGX_F64)
-      k_mspmv<double, double><<<mgrid(p.n), kMThreads, 0, s>>>(0, p.n, p.rowptr.p, p.col.p,
-                                                               p.v64.p, K, b, x, r);
-    else
-      k_mspmv<float, double><<<mgrid(p.n), kMThreads, 0, s>>>(0, p.n, p.rowptr.p, p.col.p,
-                                                              p.v32.p, K, b, x, r);
-  } else {
-    const float *v = p.storage == LGX_F32 ? p.v32.p : lv.col->pv32.p;
-    k_mspmv<float, float><<<mgrid(p.n), kMThreads, 0, s>>>(0, p.n, p.rowptr.p, p.col.p, v, K, b,
-                                                           x, r);
+    if (p.storage == LGX_F64) {
+      k_mspmv<double, double><<<mgrid(p.n), kMThreads, 0, s>>>(
+        0, p.n, p.rowptr.p, p.col.p, p.v64.p, rows, K, up, bb, x, r);
+      LGX_LAUNCH_CHECK();
+      return LGX_OK;
+    }
   }
+  const float *v = p.storage == LGX_F32 ? p.v32.p : c.pv32.p;
+  k_mspmv<float, XT><<<mgrid(p.n), kMThreads, 0, s>>>(0, p.n, p.rowptr.p, p.col.p, v, rows, K, up,
+                                                      bb, x, r);
   LGX_LAUNCH_CHECK();
   return LGX_OK;
 }
@@ -301,7 +317,7 @@ static lgx_status m_vcycle(const lgx_amg &h, int K, MWork<XT> &w, const XT *b0, 
     const lgx_amg_level &lv = *h.lv[l];
     if (lv.a->n == 0) continue;
     LGX_CHECK(m_level_sor<XT>(h, lv, K, 1, 1, bv(l), xv(l), s));
-    LGX_CHECK(m_level_residual<XT>(lv, K, bv(l), xv(l), w.r[l].p, s));
+    LGX_CHECK(m_level_residual<XT>(h, lv, K, bv(l), xv(l), w.r[l].p, s));
     const int64_t nc = h.lv[l + 1]->a->n;
     if (nc) {
       k_mrestrict<XT><<<mgrid(nc), kMThreads, 0, s>>>(nc, lv.rptr.p, lv.rlist.p, K, w.r[l].p,
@@ -452,8 +468,8 @@ static lgx_status pcg_multi(const lgx_matrix *a, lgx_amg &h, int K, const double
   const int64_t n = a->n;
   const int64_t L = (int64_t)h.lv.size();
   const bool permuted = L > 1;
-  const Csr &A = permuted ? h.lv[0]->col->pcsr : a->csr;
-  const int32_t *perm = permuted ? h.lv[0]->col->perm.p : nullptr;
+  const int32_t *perm = permuted ? h.lv[0]->perm() : nullptr;
+  const Csr &A = perm ? h.lv[0]->col->pcsr : a->csr;  // (the hierarchy's own, checked)
   const int64_t nk = n * K;
   // the stream every launch below goes to: the caller's, or the capture
   // stream while an iteration is recorded
@@ -503,10 +519,10 @@ static lgx_status pcg_multi(const lgx_matrix *a, lgx_amg &h, int K, const double
   auto apply = [&](const double *bb, const double *x, double *y) -> lgx_status {
     if (A.storage == LGX_F64)
       k_mspmv<double, double><<<mgrid(n), kMThreads, 0, s>>>(0, n, A.rowptr.p, A.col.p, A.v64.p,
-                                                             K, bb, x, y);
+                                                             nullptr, K, 0, bb, x, y);
     else
       k_mspmv<float, double><<<mgrid(n), kMThreads, 0, s>>>(0, n, A.rowptr.p, A.col.p, A.v32.p,
-                                                            K, bb, x, y);
+                                                            nullptr, K, 0, bb, x, y);
     LGX_LAUNCH_CHECK();
     return LGX_OK;
   };

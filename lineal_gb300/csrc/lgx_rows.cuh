@@ -147,12 +147,38 @@ __device__ __forceinline__ void issue_tile(const int64_t *rowptr, const int32_t 
   if (vb) bulk_g2s(st.val, val + v0, vb, bar);
 }
 
+// whether an operation names the vector rows of its matrix rows in a list
+template <class Op, class = void>
+struct RowList {
+  static constexpr bool value = false;
+};
+template <class Op>
+struct RowList<Op, std::enable_if_t<Op::kList>> {
+  static constexpr bool value = true;
+};
+// the vector row of matrix row r (in range), loaded ahead of the row
+template <class Op>
+__device__ __forceinline__ int32_t list_row(const Op &op, int64_t r, bool in) {
+  if constexpr (RowList<Op>::value) {
+    if (op.rows && in) return __ldg(op.rows + r);
+  }
+  return (int32_t)r;
+}
+template <int W, bool FLAT, class Op, typename VT>
+__device__ __forceinline__ double run_row(const Op &op, int64_t r, int32_t i, const int32_t *c,
+                                          const VT *v, int len) {
+  if constexpr (RowList<Op>::value) return op.template row<W, FLAT>(r, i, c, v, len);
+  else return op.template row<W, FLAT>(r, c, v, len);
+}
+
 // Op interface:
 //   using X = <type of the gathered vector entries>;
 //   template <int W, bool FLAT> __device__ double row(int64_t row, const int32_t *c,
 //                                                     const VT *v, int len) const;
 //     (returns the row's contribution to an optional sum; W = entries whose
 //     gathers are issued together; FLAT: products without branches, row_dot)
+//   static constexpr bool kList;  const int32_t *rows;  (kList: matrix row r is
+//     vector row rows[r], r itself when rows is null; row() takes both)
 //   static constexpr bool kReduce;  __device__ void finish(double total) const;
 //   double *partials; unsigned *counter;  (when kReduce)
 template <typename VT, class Op, int KIND>
@@ -236,12 +262,14 @@ __global__ void __launch_bounds__(kTileRows, RowCfg<VT, KIND>::ctas_per_sm)
       if (row < cur.r1) {
         const Stage<VT> sg = stage(s);
         const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
-        contrib += op.template row<RowCfg<VT, KIND>::gather, false>(row, sg.col + (b - c0), sg.val + (b - v0),
-                                                             (int)(e - b));
+        contrib += run_row<RowCfg<VT, KIND>::gather, false>(op, row, list_row(op, row, true),
+                                                            sg.col + (b - c0), sg.val + (b - v0),
+                                                            (int)(e - b));
       }
     } else if (row < cur.r1) {
       const int64_t b = rowptr[row], e = rowptr[row + 1];
-      contrib += op.template row<RowCfg<VT, KIND>::gather, false>(row, col + b, val + b, (int)(e - b));
+      contrib += run_row<RowCfg<VT, KIND>::gather, false>(op, row, list_row(op, row, true),
+                                                          col + b, val + b, (int)(e - b));
     }
     __syncthreads();
     if (NST == 1 && threadIdx.x == 0 && t + G < ntiles) {
@@ -341,6 +369,7 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
           const int32_t *__restrict__ col, const VT *__restrict__ val, Op op, int *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int W = WrowsBounds<WPC, typename Op::X, MB>::gather;
+  constexpr bool FLAT = WrowsBounds<WPC, typename Op::X, MB>::flat;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t sb = wstage_bytes(capw, sizeof(VT));
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + warp * S;
@@ -391,6 +420,8 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
     }
     if (t + S * GW < ntiles) ahead = bounds(t + S * GW);
   }
+  // (constant, like the copies: the list of a tile's rows is loaded a tile ahead)
+  int32_t at = list_row(op, rb + t * kWarpTileRows + lane, rb + t * kWarpTileRows + lane < re);
   __syncwarp();
   // the matrix copies above only read constant data; vectors come after
   pdl_wait();
@@ -410,6 +441,8 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
     const int64_t r0 = rb + t * kWarpTileRows;
     const int64_t row = r0 + lane;
     const int64_t r1 = min(r0 + kWarpTileRows, re);
+    const int32_t i = at;
+    at = list_row(op, row + GW * kWarpTileRows, row + GW * kWarpTileRows < re);
     if (!unstaged[s]) {
       constexpr int64_t CA = 4, VA = 16 / (int64_t)sizeof(VT);
       const Stage<VT> sg = stage(s);
@@ -418,11 +451,12 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
       const int64_t c0 = e0 & ~(CA - 1), v0 = e0 & ~(VA - 1);
       if (row < r1) {
         const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
-        contrib += op.template row<W, WrowsBounds<WPC, typename Op::X, MB>::flat>(row, sg.col + (b - c0), sg.val + (b - v0), (int)(e - b));
+        contrib += run_row<W, FLAT>(op, row, i, sg.col + (b - c0), sg.val + (b - v0),
+                                    (int)(e - b));
       }
     } else if (row < r1) {
       const int64_t b = rowptr[row], e = rowptr[row + 1];
-      contrib += op.template row<W, WrowsBounds<WPC, typename Op::X, MB>::flat>(row, col + b, val + b, (int)(e - b));
+      contrib += run_row<W, FLAT>(op, row, i, col + b, val + b, (int)(e - b));
     }
     __syncwarp();
     if (lane == 0 && t + S * GW < ntiles) {

@@ -244,8 +244,10 @@ __global__ void k_to_f32(int64_t n, const double *src, float *dst) {
     dst[i] = (float)src[i];
 }
 
-lgx_status colouring_build(const Csr &a, const int32_t *d_colour, int32_t ncolours,
-                           cudaStream_t s, lgx_colouring &out) {
+// the colours checked and the row order they give (perm, iperm, offsets);
+// `flag` holds n int64 of scratch for the caller afterwards
+static lgx_status colouring_order(const Csr &a, const int32_t *d_colour, int32_t ncolours,
+                                  cudaStream_t s, lgx_colouring &out, DBuf<int64_t> &flag) {
   const int64_t n = a.n;
   if (ncolours < 1 && n > 0) return fail(LGX_ERR_INVALID, "colouring needs at least one colour");
   out.n = n;
@@ -257,7 +259,7 @@ lgx_status colouring_build(const Csr &a, const int32_t *d_colour, int32_t ncolou
   }
   LGX_CHECK(out.perm.alloc(n));
   LGX_CHECK(out.iperm.alloc(n));
-  DBuf<int64_t> flag, pos;
+  DBuf<int64_t> pos;
   DBuf<int> bad;
   LGX_CHECK(flag.alloc(n));
   LGX_CHECK(pos.alloc(n + 1));
@@ -287,6 +289,15 @@ lgx_status colouring_build(const Csr &a, const int32_t *d_colour, int32_t ncolou
   if (h_bad & 1) return fail(LGX_ERR_INVALID, "colour index out of range");
   if (h_bad & 2) return fail(LGX_ERR_INVALID, "adjacent rows share a colour");
   if (base != n) return fail(LGX_ERR_INVALID, "colouring does not cover every row");
+  return LGX_OK;
+}
+
+lgx_status colouring_build(const Csr &a, const int32_t *d_colour, int32_t ncolours,
+                           cudaStream_t s, lgx_colouring &out) {
+  DBuf<int64_t> flag;
+  LGX_CHECK(colouring_order(a, d_colour, ncolours, s, out, flag));
+  const int64_t n = a.n;
+  const unsigned g = (unsigned)std::min<int64_t>(grid_for(n, 256), 16384);
   // permuted CSR
   Csr &p = out.pcsr;
   p.n = n;
@@ -320,6 +331,152 @@ lgx_status colouring_build(const Csr &a, const int32_t *d_colour, int32_t ncolou
     LGX_LAUNCH_CHECK();
   }
   return csr_compute_max_window(p, s);
+}
+
+// entries of each row in earlier (lo, by colour order) and later (up, by
+// natural order) colours, and the whole row's length (by colour order)
+__global__ void k_half_count(int64_t n, const int64_t *__restrict__ rowptr,
+                             const int32_t *__restrict__ col, const int32_t *__restrict__ perm,
+                             const int32_t *__restrict__ colour, int64_t *len, int64_t *lo_len,
+                             int64_t *up_len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
+    const int64_t i = perm[r];
+    const int64_t b = rowptr[i], m = rowptr[i + 1] - b;
+    const int32_t ci = colour[i];
+    int lo = 0, up = 0;
+    for (int64_t k = lane; k < m; k += 32) {
+      const int32_t cj = colour[col[b + k]];
+      lo += cj < ci;
+      up += cj > ci;
+    }
+    lo = __reduce_add_sync(0xffffffffu, lo);
+    up = __reduce_add_sync(0xffffffffu, up);
+    if (lane == 0) {
+      len[r] = m;
+      lo_len[r] = lo;
+      up_len[i] = up;
+    }
+  }
+}
+
+template <typename T>
+struct RowsOut {
+  const int64_t *ptr;
+  int32_t *col;
+  T *val;
+};
+
+// the rows and their halves, a warp per row, entries in row order; the
+// diagonal and (FP64 values) its reciprocal as k_colour_rdiag gives them
+template <typename VT, typename OT>
+__global__ void k_half_fill(int64_t n, const int64_t *__restrict__ rowptr,
+                            const int32_t *__restrict__ col, const VT *__restrict__ val,
+                            const int32_t *__restrict__ perm, const int32_t *__restrict__ colour,
+                            RowsOut<OT> full, RowsOut<OT> lo, RowsOut<OT> up, double *pdiag,
+                            double *rdiag) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < n; r += nw) {
+    const int64_t i = perm[r];
+    const int64_t b = rowptr[i], m = rowptr[i + 1] - b;
+    const int32_t ci = colour[i];
+    int64_t o = full.ptr[r], ol = lo.ptr[r], ou = up.ptr[i];
+    for (int64_t k0 = 0; k0 < m; k0 += 32) {
+      const int64_t k = k0 + lane;
+      const bool in = k < m;
+      const int32_t c = in ? col[b + k] : 0;
+      const VT v = in ? val[b + k] : VT(0);
+      const int32_t cj = in ? colour[c] : ci;
+      const bool is_lo = cj < ci, is_up = cj > ci;
+      const unsigned ml = __ballot_sync(0xffffffffu, is_lo), mu = __ballot_sync(0xffffffffu, is_up);
+      if (in) {
+        full.col[o + k] = c;
+        full.val[o + k] = (OT)v;
+        if (c == i) {
+          const double d = (double)v;
+          pdiag[r] = d;
+          if (rdiag) {
+            const int e = (int)((__double_as_longlong(d) >> 52) & 0x7ff);
+            rdiag[r] = (e > 1023 - 400 && e < 1023 + 400) ? 1.0 / d : 0.0;
+          }
+        }
+      }
+      if (is_lo) {
+        const int64_t at = ol + __popc(ml & below);
+        lo.col[at] = c;
+        lo.val[at] = (OT)v;
+      }
+      if (is_up) {
+        const int64_t at = ou + __popc(mu & below);
+        up.col[at] = c;
+        up.val[at] = (OT)v;
+      }
+      ol += __popc(ml);
+      ou += __popc(mu);
+    }
+  }
+}
+
+template <typename OT>
+static RowsOut<OT> rows_out(Csr &a) {
+  if constexpr (sizeof(OT) == 8) return {a.rowptr.p, a.col.p, a.v64.p};
+  else return {a.rowptr.p, a.col.p, a.v32.p};
+}
+
+lgx_status colouring_build_natural(const Csr &a, const int32_t *d_colour, int32_t ncolours,
+                                   bool f32, cudaStream_t s, lgx_colouring &out) {
+  DBuf<int64_t> len, lo_len, up_len;
+  LGX_CHECK(colouring_order(a, d_colour, ncolours, s, out, len));
+  const int64_t n = a.n;
+  const lgx_dtype storage = f32 ? LGX_F32 : a.storage;
+  out.natural = true;
+  LGX_CHECK(lo_len.alloc(n));
+  LGX_CHECK(up_len.alloc(n));
+  // a warp per row
+  const unsigned g = (unsigned)std::min<int64_t>(grid_for(std::max<int64_t>(n, 1) * 32, 256), 16384);
+  if (n > 0) {
+    k_half_count<<<g, 256, 0, s>>>(n, a.rowptr.p, a.col.p, out.perm.p, out.colour.p, len.p,
+                                   lo_len.p, up_len.p);
+    LGX_LAUNCH_CHECK();
+  }
+  Csr *list[3] = {&out.pcsr, &out.lo, &out.up};
+  const int64_t *lens[3] = {len.p, lo_len.p, up_len.p};
+  int64_t nnz[3] = {0, 0, 0};
+  for (int k = 0; k < 3; ++k) {
+    list[k]->n = n;
+    list[k]->symmetric = k == 0 ? a.symmetric : 0;
+    list[k]->storage = storage;
+    LGX_CHECK(list[k]->rowptr.alloc(n + 3));  // +2: staged row-offset spans
+    LGX_CHECK(inclusive_offsets(n, lens[k], list[k]->rowptr.p, s));
+    LGX_CUDA(cudaMemcpyAsync(&nnz[k], list[k]->rowptr.p + n, sizeof(int64_t),
+                             cudaMemcpyDeviceToHost, s));
+  }
+  LGX_CHECK(csr_compute_extents(list, 3, s));  // synchronises: nnz has arrived
+  for (int k = 0; k < 3; ++k) {
+    list[k]->nnz = nnz[k];
+    LGX_CHECK(csr_alloc_arrays(*list[k], nnz[k], storage));
+  }
+  if (n == 0) return LGX_OK;
+  LGX_CHECK(out.pdiag.alloc(n));
+  if (storage == LGX_F64) {
+    LGX_CHECK(out.rdiag.alloc(n));
+    k_half_fill<double, double><<<g, 256, 0, s>>>(
+      n, a.rowptr.p, a.col.p, a.v64.p, out.perm.p, out.colour.p, rows_out<double>(out.pcsr),
+      rows_out<double>(out.lo), rows_out<double>(out.up), out.pdiag.p, out.rdiag.p);
+  } else if (a.storage == LGX_F64) {
+    k_half_fill<double, float><<<g, 256, 0, s>>>(
+      n, a.rowptr.p, a.col.p, a.v64.p, out.perm.p, out.colour.p, rows_out<float>(out.pcsr),
+      rows_out<float>(out.lo), rows_out<float>(out.up), out.pdiag.p, nullptr);
+  } else {
+    k_half_fill<float, float><<<g, 256, 0, s>>>(
+      n, a.rowptr.p, a.col.p, a.v32.p, out.perm.p, out.colour.p, rows_out<float>(out.pcsr),
+      rows_out<float>(out.lo), rows_out<float>(out.up), out.pdiag.p, nullptr);
+  }
+  LGX_LAUNCH_CHECK();
+  return LGX_OK;
 }
 
 lgx_status colouring_make_f32(lgx_colouring &c, cudaStream_t s) {
@@ -373,6 +530,24 @@ lgx_status colouring_make_bf16(lgx_colouring &c, cudaStream_t s) {
 // With rdiag (FP64 values and vectors) the regular row divides through the
 // reciprocal table (same quotient), and relax == 1 skips the (1 - relax) x_i
 // term where it cannot change the result (q nonzero, x_i finite).
+// accum / diag by the row's formula, the sweep's last step: x_i from the
+// accumulated sum, with y the reciprocal table's entry (0: divide)
+template <typename XT>
+__device__ __forceinline__ XT sor_value(XT accum, XT diag, XT xi, double y, XT relax, XT m1,
+                                        int ultra, int relax_one) {
+  if (ultra) return xi + relax * accum / fabs(diag);
+  XT quot;
+  if constexpr (sizeof(XT) == 8) {
+    quot = (nonzero_bits(y) && exponent_within_400(accum)) ? div_by_recip(accum, diag, y)
+                                                           : accum / diag;
+    // fma(1, q, 0 * x_i) == q for nonzero q and finite x_i
+    if (relax_one && nonzero_bits(quot) && exponent_field(xi) != 0x7ff) return quot;
+  } else {
+    quot = accum / diag;
+  }
+  return fma(relax, quot, m1 * xi);
+}
+
 template <typename VT, typename XT>
 struct SorOp {
   const XT *b;
@@ -386,13 +561,16 @@ struct SorOp {
   int from_zero = 0;
   int64_t visit_end = 0;
   const float *scale = nullptr;  // bfloat16 values: row factor (the diagonal)
+  const int32_t *rows = nullptr;  // natural-order levels: vector row of each matrix row
   using X = XT;
   static constexpr bool kReduce = false;
+  static constexpr bool kList = true;
   static constexpr int kTuneClass = 1;
   double *partials = nullptr;
   unsigned *counter = nullptr;
   template <int W, bool FLAT>
-  __device__ __forceinline__ double row(int64_t i, const int32_t *c, const VT *v, int len) const {
+  __device__ __forceinline__ double row(int64_t r, int32_t i, const int32_t *c, const VT *v,
+                                        int len) const {
     if constexpr (kIsBf16<VT>) {
       return row_scaled<W>(i, c, v, len);
     }
@@ -400,7 +578,7 @@ struct SorOp {
     const XT xi = from_zero ? XT(0) : x[i];
     const int64_t end = from_zero ? visit_end : INT64_MAX;
     // constant, so it loads with the row's first loads
-    const double y = sizeof(XT) == 8 && rdiag ? rdiag[i] : 0.0;
+    const double y = sizeof(XT) == 8 && rdiag ? rdiag[r] : 0.0;
     for (int k = 0; k < len; k += W) {
       const int m = len - k;
       int32_t cc[W];
@@ -421,22 +599,7 @@ struct SorOp {
         }
       }
     }
-    if (ultra) {
-      x[i] = xi + relax * accum / fabs(diag);
-      return 0.0;
-    }
-    XT quot;
-    if constexpr (sizeof(XT) == 8) {
-      quot = (nonzero_bits(y) && exponent_within_400(accum)) ? div_by_recip(accum, diag, y)
-                                                             : accum / diag;
-      if (relax_one && nonzero_bits(quot) && exponent_field(xi) != 0x7ff) {
-        x[i] = quot;  // fma(1, q, 0 * x_i) == q for nonzero q and finite x_i
-        return 0.0;
-      }
-    } else {
-      quot = accum / diag;
-    }
-    x[i] = fma(relax, quot, m1 * xi);
+    x[i] = sor_value<XT>(accum, diag, xi, y, relax, m1, ultra, relax_one);
     return 0.0;
   }
   // bfloat16 values v with a_ij = s_i v_ij: accum = b_i - s_i sum_{j != i} v_ij x_j,
@@ -481,6 +644,67 @@ struct SorOp {
   __device__ __forceinline__ void finish(double) const {}
 };
 
+// One colour of a forward sweep from x = 0 on the rows' earlier-colour halves
+// (lgx_colouring::lo): what SorOp does with the entries of colours not yet
+// visited reading 0, whose products leave the sum as it is.
+template <typename VT, typename XT>
+struct SorLoOp {
+  const XT *b;
+  XT *x;
+  XT relax, m1;
+  int ultra, relax_one;
+  const double *pdiag, *rdiag;
+  const int32_t *rows;
+  using X = XT;
+  static constexpr bool kReduce = false;
+  static constexpr bool kList = true;
+  static constexpr int kTuneClass = 1;
+  double *partials = nullptr;
+  unsigned *counter = nullptr;
+  template <int W, bool FLAT>
+  __device__ __forceinline__ double row(int64_t r, int32_t i, const int32_t *c, const VT *v,
+                                        int len) const {
+    const double y = sizeof(XT) == 8 && rdiag ? rdiag[r] : 0.0;
+    const XT diag = (XT)pdiag[r];
+    XT accum = b[i];
+    for (int k = 0; k < len; k += W) {
+      const int m = len - k;
+      int32_t cc[W];
+      XT xv[W];
+      row_columns<W>(c, k, len, cc);
+#pragma unroll
+      for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], u < m);
+#pragma unroll
+      for (int u = 0; u < W; ++u)
+        if (u < m) accum = fma(-cvt<XT>(v[k + u]), xv[u], accum);
+    }
+    x[i] = sor_value<XT>(accum, diag, XT(0), y, relax, m1, ultra, relax_one);
+    return 0.0;
+  }
+  __device__ __forceinline__ void finish(double) const {}
+};
+
+// r = -U x (mc_up_residual) / r = b - A x on listed rows (mc_residual)
+template <typename VT, typename XT, bool UP>
+struct ListResidualOp {
+  const XT *b, *x;
+  XT *r;
+  const int32_t *rows;
+  using X = XT;
+  static constexpr bool kReduce = false;
+  static constexpr bool kList = true;
+  double *partials = nullptr;
+  unsigned *counter = nullptr;
+  template <int W, bool FLAT>
+  __device__ __forceinline__ double row(int64_t, int32_t i, const int32_t *c, const VT *v,
+                                        int len) const {
+    const XT ax = row_dot<W, FLAT, VT, XT>(c, v, len, x, XT(0));
+    r[i] = UP ? -ax : b[i] - ax;
+    return 0.0;
+  }
+  __device__ __forceinline__ void finish(double) const {}
+};
+
 // First colour of a forward sweep from x = 0: every neighbour still reads 0,
 // so the row's products with them leave accum = b_i (an fma with a zero
 // product; where only the sign of a zero could differ, the row's result is
@@ -489,38 +713,24 @@ struct SorOp {
 template <typename VT, typename XT>
 __global__ void k_sor_first_colour(int64_t rb, int64_t re, const double *__restrict__ pdiag,
                                    const double *__restrict__ rdiag,
-                                   const float *__restrict__ scale, const XT *__restrict__ b,
+                                   const float *__restrict__ scale,
+                                   const int32_t *__restrict__ rows, const XT *__restrict__ b,
                                    XT *__restrict__ x, XT relax, XT m1, int ultra,
                                    int relax_one) {
   pdl_trigger();
   pdl_wait();
-  for (int64_t i = rb + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < re;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t r = rb + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < re;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = rows ? rows[r] : r;
     const XT accum = b[i];
     XT diag;
     if constexpr (kIsBf16<VT>) {
       diag = scale[i];  // s_i * v_ii with v_ii = 1 (scaled by the diagonal)
     } else {
-      diag = (XT)pdiag[i];
+      diag = (XT)pdiag[r];
     }
-    const XT xi = XT(0);
-    if (ultra) {
-      x[i] = xi + relax * accum / fabs(diag);
-      continue;
-    }
-    XT quot;
-    if constexpr (sizeof(XT) == 8 && !kIsBf16<VT>) {
-      const double y = rdiag ? rdiag[i] : 0.0;
-      quot = (nonzero_bits(y) && exponent_within_400(accum)) ? div_by_recip(accum, diag, y)
-                                                             : accum / diag;
-      if (relax_one && nonzero_bits(quot)) {
-        x[i] = quot;
-        continue;
-      }
-    } else {
-      quot = accum / diag;
-    }
-    x[i] = fma(relax, quot, m1 * xi);
+    const double y = sizeof(XT) == 8 && !kIsBf16<VT> && rdiag ? rdiag[r] : 0.0;
+    x[i] = sor_value<XT>(accum, diag, XT(0), y, relax, m1, ultra, relax_one);
   }
 }
 
@@ -532,6 +742,9 @@ lgx_status mc_sor_sweep(const lgx_colouring &c, const VT *val, double relax, int
   const Csr &p = c.pcsr;
   SorOp<VT, XT> op{b, x, (XT)relax, XT(1) - (XT)relax, ultra};
   op.scale = scale;
+  op.rows = c.natural ? c.perm.p : nullptr;
+  if (kIsBf16<VT> && c.natural)
+    return fail(LGX_ERR_UNSUPPORTED, "natural-order levels have no bfloat16 values");
   if (kIsBf16<VT> && !scale) return fail(LGX_ERR_INVALID, "bfloat16 values need row scales");
   if constexpr (sizeof(VT) == 8 && sizeof(XT) == 8) {
     op.rdiag = c.rdiag.p;
@@ -549,12 +762,27 @@ lgx_status mc_sor_sweep(const lgx_colouring &c, const VT *val, double relax, int
         LGX_CUDA(launch_pdl(sizeof(XT) == 4 || re - rb <= pdl_fp64_rows(),
                             k_sor_first_colour<VT, XT>, dim3(g), dim3(256), 0,
                             s, rb, re, (const double *)c.pdiag.p, (const double *)op.rdiag,
-                            scale, b, x, op.relax, op.m1, ultra, op.relax_one));
+                            scale, op.rows, b, x, op.relax, op.m1, ultra, op.relax_one));
         count_launch();
       }
       continue;
     }
-    op.visit_end = rb;  // forward: exactly the rows before this colour are visited
+    if constexpr (!kIsBf16<VT>) {
+      if (op.from_zero && c.lo.n > 0) {
+        // half the entries of the row
+        const VT *lv;
+        if constexpr (sizeof(VT) == 8) lv = c.lo.v64.p;
+        else lv = c.lo.v32.p;
+        LGX_CHECK(launch_rows<VT>(rb, re, c.lo, lv,
+                                  SorLoOp<VT, XT>{b, x, op.relax, op.m1, ultra, op.relax_one,
+                                                  c.pdiag.p, op.rdiag, op.rows},
+                                  s));
+        continue;
+      }
+    }
+    // forward: exactly the rows before this colour are visited (a natural-order
+    // level has its halves for sweeps from zero)
+    op.visit_end = rb;
     // the last colour of a forward sweep on grid rows can also leave its
     // rows' residuals in r_last
     const bool with_res = r_last && res_from && forward && k == c.ncolours - 1 && re > rb &&
@@ -571,6 +799,30 @@ lgx_status mc_sor_sweep(const lgx_colouring &c, const VT *val, double relax, int
   }
   return LGX_OK;
 }
+
+template <typename VT, typename XT>
+lgx_status mc_residual(const lgx_colouring &c, const VT *val, const XT *b, const XT *x, XT *r,
+                       cudaStream_t s) {
+  return launch_rows<VT>(0, c.n, c.pcsr, val, ListResidualOp<VT, XT, false>{b, x, r, c.perm.p}, s);
+}
+
+template <typename VT, typename XT>
+lgx_status mc_up_residual(const lgx_colouring &c, const XT *x, XT *r, cudaStream_t s) {
+  const VT *v;
+  if constexpr (sizeof(VT) == 8) v = c.up.v64.p;
+  else v = c.up.v32.p;
+  return launch_rows<VT>(0, c.n, c.up, v, ListResidualOp<VT, XT, true>{nullptr, x, r, nullptr}, s);
+}
+
+#define LGX_MC_RESIDUAL(VT, XT)                                                              \
+  template lgx_status mc_residual<VT, XT>(const lgx_colouring &, const VT *, const XT *,     \
+                                          const XT *, XT *, cudaStream_t);                   \
+  template lgx_status mc_up_residual<VT, XT>(const lgx_colouring &, const XT *, XT *,        \
+                                             cudaStream_t);
+LGX_MC_RESIDUAL(double, double)
+LGX_MC_RESIDUAL(float, double)
+LGX_MC_RESIDUAL(float, float)
+#undef LGX_MC_RESIDUAL
 
 template lgx_status mc_sor_sweep<double, double>(const lgx_colouring &, const double *, double,
                                                  int, int, const double *, double *,

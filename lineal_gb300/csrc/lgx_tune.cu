@@ -148,6 +148,13 @@ int cycle_value_bytes(const lgx_amg &h, const lgx_colouring &c) {
   return h.p.cycle_bf16 ? 2 : 4;
 }
 
+// a level's slot of an operation class and value type, in every matrix that
+// its operation of that class reads
+void set_slot(lgx_colouring &c, int op, int vi, int8_t cfg) {
+  c.pcsr.tuned[op][vi] = cfg;
+  if (c.natural) (op == 0 ? c.up : c.lo).tuned[op][vi] = cfg;
+}
+
 // One V-cycle (zero right-hand side; the work does not depend on values),
 // recorded and replayed: minimum of three timed replays.
 lgx_status time_cycle(lgx_amg &h, TuneObjects &o, const double *b, double *x, int reps,
@@ -176,7 +183,7 @@ lgx_status confirm_in_cycle(lgx_amg &h, std::vector<lgx_tune_entry> &all, int re
   for (int l = 0; l + 1 < L; ++l) {
     lgx_amg_level &lv = *h.lv[l];
     if (!lv.col) continue;
-    Csr &p = lv.col->pcsr;
+    lgx_colouring &p = *lv.col;
     const int vb = cycle_value_bytes(h, *lv.col);
     const int vi = vb == 8 ? 0 : vb == 4 ? 1 : 2;
     std::vector<lgx_tune_entry *> changed;
@@ -186,10 +193,10 @@ lgx_status confirm_in_cycle(lgx_amg &h, std::vector<lgx_tune_entry> &all, int re
     if (changed.empty()) continue;
     float t_win = 0.f, t_def = 0.f;
     LGX_CHECK(time_cycle(h, o, b.p, x.p, reps, s, &t_win));
-    for (auto *e : changed) p.tuned[e->op][vi] = -1;
+    for (auto *e : changed) set_slot(p, e->op, vi, -1);
     LGX_CHECK(time_cycle(h, o, b.p, x.p, reps, s, &t_def));
     if (t_win < t_def) {
-      for (auto *e : changed) p.tuned[e->op][vi] = (int8_t)e->config;
+      for (auto *e : changed) set_slot(p, e->op, vi, (int8_t)e->config);
     } else {
       for (auto *e : changed) e->config = def;
     }
@@ -221,15 +228,28 @@ lgx_status tune_level(lgx_colouring &c, const VT *val, const float *scale, doubl
   LGX_CHECK(v.alloc(p.n, s));
   const int vi = tune_value_index<VT>();
   lgx_tune_entry e = blank_entry(level, 0, (int)sizeof(VT));
-  LGX_CHECK(tune_slot(p.tuned[0][vi], reps, s, e, [&](cudaStream_t cs) {
-    return csr_residual<VT, XT>(p, val, v.b.p, v.x.p, v.r.p, nullptr, nullptr, nullptr, cs,
-                                scale);
-  }));
+  if constexpr (!kIsBf16<VT>) {
+    if (c.natural) {
+      // the cycle's residual: the rows' later-colour halves (relax 1), or whole
+      const bool up = relax == 1.0 && !ultra;
+      LGX_CHECK(tune_slot((up ? c.up : p).tuned[0][vi], reps, s, e, [&](cudaStream_t cs) {
+        return up ? mc_up_residual<VT, XT>(c, v.x.p, v.r.p, cs)
+                  : mc_residual<VT, XT>(c, val, v.b.p, v.x.p, v.r.p, cs);
+      }));
+      set_slot(c, 0, vi, (int8_t)e.config);
+    }
+  }
+  if (!c.natural)
+    LGX_CHECK(tune_slot(p.tuned[0][vi], reps, s, e, [&](cudaStream_t cs) {
+      return csr_residual<VT, XT>(p, val, v.b.p, v.x.p, v.r.p, nullptr, nullptr, nullptr, cs,
+                                  scale);
+    }));
   out.push_back(e);
   e = blank_entry(level, 1, (int)sizeof(VT));
   LGX_CHECK(tune_slot(p.tuned[1][vi], reps, s, e, [&](cudaStream_t cs) {
     return mc_sor_sweep<VT, XT>(c, val, relax, 1, ultra, v.b.p, v.x.p, cs, 0, scale);
   }));
+  set_slot(c, 1, vi, (int8_t)e.config);
   out.push_back(e);
   return LGX_OK;
 }
@@ -288,8 +308,18 @@ lgx_status lgx_amg_autotune(lgx_amg *h, int reps, lgx_tune_entry *out, int max_o
     // grid level runs its own kernels, not the row engine
     if (!lv.col || l == L - 1 || lv.col->pcsr.n == 0 || lv.col->pcsr.grid) continue;
     lgx_colouring &c = *lv.col;
-    if (l == 0 && c.pcsr.storage == LGX_F64 && h->f32)
-      LGX_CHECK(tune_product64(c.pcsr, 0, reps, s, all));
+    if (l == 0 && lv.a->storage == LGX_F64 && h->f32) {
+      if (!c.natural) {
+        LGX_CHECK(tune_product64(c.pcsr, 0, reps, s, all));
+      } else {
+        // the caller's matrix itself: a choice it already made stays
+        Csr &a = const_cast<Csr &>(*lv.a);
+        const int8_t own = h->tuned_outer ? (int8_t)-1 : a.tuned[0][0];
+        LGX_CHECK(tune_product64(a, 0, reps, s, all));
+        if (own >= 0) a.tuned[0][0] = own;
+        else h->tuned_outer = true;
+      }
+    }
     if (!h->f32) {
       if (c.pcsr.storage == LGX_F64)
         LGX_CHECK((tune_level<double, double>(c, c.pcsr.v64.p, nullptr, relax, ultra, l, reps, s,
@@ -313,7 +343,11 @@ lgx_status lgx_amg_autotune_reset(lgx_amg *h) {
   if (!h) return fail(LGX_ERR_INVALID, "null hierarchy");
   for (auto &lv : h->lv)
     if (lv->col)
-      for (auto &cls : lv->col->pcsr.tuned)
-        for (auto &slot : cls) slot = -1;
+      for (int op = 0; op < 2; ++op)
+        for (int vi = 0; vi < 3; ++vi) set_slot(*lv->col, op, vi, -1);
+  if (h->tuned_outer) {
+    const_cast<Csr &>(*h->lv[0]->a).tuned[0][0] = -1;
+    h->tuned_outer = false;
+  }
   return LGX_OK;
 }
