@@ -28,6 +28,11 @@ const float *amg_finest_values_f32(const lgx_amg &h);
 
 namespace lgx {
 
+// a whole solve in one launch (lgx_solo.cu), where it takes it
+lgx_status solo_solve(bool cg, const lgx_matrix *a, const double *d_b, double *d_x,
+                      const lgx_solve_params *p, cudaStream_t s, int64_t *iterations,
+                      double *final_rel, double *history, bool *done);
+
 struct KScalars {
   double rho, rho_old, alpha, beta, omega, res2, den, tmp;
   int flag;  // bit 0: breakdown, bit 1: non-finite
@@ -614,6 +619,10 @@ static lgx_status krylov_create(int kind, const lgx_matrix *a, const double *d_b
 static lgx_status run_solve(int kind, const lgx_matrix *a, const double *d_b, double *d_x,
                             const lgx_solve_params *p, cudaStream_t s, int64_t *iterations,
                             double *final_rel, double *history) {
+  bool done = false;
+  const lgx_status solo = solo_solve(kind == LGX_KRYLOV_CG, a, d_b, d_x, p, s, iterations,
+                                     final_rel, history, &done);
+  if (done || solo != LGX_OK) return solo;
   std::unique_ptr<lgx_krylov> K;
   LGX_CHECK(krylov_create(kind, a, d_b, d_x, p, s, K));
   if (history) history[0] = K->r0;
