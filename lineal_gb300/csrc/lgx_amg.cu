@@ -2314,16 +2314,20 @@ __global__ void k_rlist_fill(int64_t nc, const int32_t *perm_c, const int64_t *l
 }
 
 // coarse b[I'] = sum over the aggregate's fine rows (list order) of r
-// (vector-shared.hpp:49-56)
+// (vector-shared.hpp:49-56); fine rows at or after zero_from hold 0 and are not
+// read
 template <typename XT>
 __global__ void k_restrict(int64_t nc, const int64_t *rptr, const int32_t *rlist,
-                           const XT *__restrict__ r, XT *__restrict__ bc) {
+                           int64_t zero_from, const XT *__restrict__ r, XT *__restrict__ bc) {
   pdl_trigger();
   pdl_wait();
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < nc;
        c += (int64_t)gridDim.x * blockDim.x) {
     XT s = XT(0);
-    for (int64_t k = rptr[c]; k < rptr[c + 1]; ++k) s = s + r[rlist[k]];
+    for (int64_t k = rptr[c]; k < rptr[c + 1]; ++k) {
+      const int64_t i = rlist[k];
+      if (i < zero_from) s = s + r[i];
+    }
     bc[c] = s;
   }
 }
@@ -2719,6 +2723,20 @@ static lgx_status level_sor(lgx_amg_level &lv, const lgx_amg &h, int forward, co
   }
 }
 
+// Every residual of the cycle follows a forward sweep from zero: with relax 1 it
+// is -U x (mc_up_residual).
+static bool up_residual(const lgx_amg &h, const lgx_amg_level &lv) {
+  return h.p.smoother_relax == 1.0 && !h.p.smoother_ultra && !lv.stencil &&
+         !(h.f32 && h.p.cycle_bf16);
+}
+
+// the first row that such a residual leaves unwritten (its residual is 0)
+static int64_t residual_zero_from(const lgx_amg &h, const lgx_amg_level &lv) {
+  const lgx_colouring &c = *lv.col;
+  return up_residual(h, lv) && !c.natural && c.ncolours > 0 ? c.offsets[c.ncolours - 1]
+                                                            : INT64_MAX;
+}
+
 // The residual of rows [0, rend) of a level whose sweep left the residuals
 // of its last colour (rows rend on) already; the whole residual when rend
 // is the level's size.
@@ -2736,15 +2754,15 @@ static lgx_status level_residual(lgx_amg_level &lv, const lgx_amg &h, const XT *
     else
       return fail(LGX_ERR_UNSUPPORTED, "a stencil finest level runs the FP64 cycle");
   }
-  if (c.natural) {
-    // every residual of the cycle follows a forward sweep from zero
-    const bool up = h.p.smoother_relax == 1.0 && !h.p.smoother_ultra;
+  const bool up = up_residual(h, lv);
+  if (c.natural || up) {
     if constexpr (sizeof(XT) == 8)
       if (c.pcsr.storage == LGX_F64)
-        return up ? mc_up_residual<double, double>(c, x, r, s)
+        return up ? mc_up_residual<double, double>(c, c.pcsr.v64.p, x, r, s)
                   : mc_residual<double, double>(c, c.pcsr.v64.p, b, x, r, s);
-    return up ? mc_up_residual<float, XT>(c, x, r, s)
-              : mc_residual<float, XT>(c, c.pcsr.v32.p, b, x, r, s);
+    const float *v = c.pcsr.storage == LGX_F32 ? c.pcsr.v32.p : c.pv32.p;
+    return up ? mc_up_residual<float, XT>(c, v, x, r, s)
+              : mc_residual<float, XT>(c, v, b, x, r, s);
   }
   if constexpr (sizeof(XT) == 8) {
     if (c.pcsr.storage == LGX_F64)
@@ -2815,12 +2833,13 @@ static lgx_status vcycle_impl(lgx_amg &h, const XT *b0, XT *x0, cudaStream_t s) 
     XT *x = l == 0 ? x0 : level_vec<XT>(lv, 1);
     const int64_t n = lv.a->n;
     if (n == 0) continue;
-    // forward sweep from x = 0; its last colour, on float 7-point grid rows,
-    // also leaves its rows' residuals, so the residual pass covers the rows
-    // before it
+    // forward sweep from x = 0; its last colour, on float 7-point grid rows with
+    // relax other than 1, also leaves its rows' residuals, so the residual pass
+    // covers the rows before it
     XT *r = level_vec<XT>(lv, 2);
     int64_t res_from = n;
-    LGX_CHECK(level_sor<XT>(lv, h, 1, b, x, s, 1, fused_residual_enabled() ? r : nullptr,
+    LGX_CHECK(level_sor<XT>(lv, h, 1, b, x, s, 1,
+                            fused_residual_enabled() && !up_residual(h, lv) ? r : nullptr,
                             &res_from));
     LGX_CHECK(level_residual_part<XT>(lv, h, b, x, r, res_from, s));
     lgx_amg_level &cv = *h.lv[l + 1];
@@ -2829,7 +2848,8 @@ static lgx_status vcycle_impl(lgx_amg &h, const XT *b0, XT *x0, cudaStream_t s) 
       LGX_CUDA(launch_pdl(sizeof(XT) == 4 || nc <= pdl_fp64_rows(), k_restrict<XT>,
                           dim3(std::min<int64_t>(grid_for(nc, 128), 65535)),
                           dim3(128), 0, s, nc, (const int64_t *)lv.rptr.p,
-                          (const int32_t *)lv.rlist.p, (const XT *)level_vec<XT>(lv, 2),
+                          (const int32_t *)lv.rlist.p, residual_zero_from(h, lv),
+                          (const XT *)level_vec<XT>(lv, 2),
                           level_vec<XT>(cv, 0)));
       count_launch();
     }

@@ -349,12 +349,15 @@ struct G27Row {
 
 // x of neighbour c for entry e of a row (0 for unvisited colours in a
 // forward sweep from zero; the diagonal's x is not read here)
-template <typename XT, int MODE, int PTS>
+template <typename VT, typename XT, int MODE, int PTS>
 __device__ __forceinline__ XT g27_x(const XT *x, int64_t c, int e, const G27Sor &so) {
   if (g_sor_mode<MODE>() && e == g_diag<PTS>()) return XT(0);
   // the load stays unconditional (a round's loads go out together)
   const XT xl = g27_ld(x + c);
-  return (g_sor_mode<MODE>() && ((so.fz_mask >> e) & 1u)) ? XT(0) : xl;
+  // (other sweeps from zero run on half rows)
+  if constexpr (MODE == 4 || (MODE == 2 && kIsBf16<VT>))
+    if ((so.fz_mask >> e) & 1u) return XT(0);
+  return xl;
 }
 
 // one row per thread
@@ -381,7 +384,7 @@ __global__ void __launch_bounds__(256)
       const int e = e0 + u;
       if (e >= PTS) break;
       av[u] = cvt<XT>(g27_ld(v + (int64_t)e * g.stride + r));
-      xv[u] = g27_x<XT, MODE, PTS>(x, g_in<PTS>(sides, e) ? g_nb<PTS>(g, cell, r, e) : r, e, so);
+      xv[u] = g27_x<VT, XT, MODE, PTS>(x, g_in<PTS>(sides, e) ? g_nb<PTS>(g, cell, r, e) : r, e, so);
     }
 #pragma unroll
     for (int u = 0; u < B; ++u) {
@@ -476,7 +479,7 @@ __global__ void __launch_bounds__(256)
       g27_ldv<VT, R>(v + (int64_t)e * g.stride + r0, av[u]);
 #pragma unroll
       for (int q = 0; q < R; ++q)
-        xv[u][q] = g27_x<float, MODE, PTS>(
+        xv[u][q] = g27_x<VT, float, MODE, PTS>(
           x, g_in<PTS>(sides[q], e) ? g_nb<PTS>(g, cell[q], r0 + q, e) : r0 + q, e, so);
     }
 #pragma unroll
@@ -605,6 +608,191 @@ __global__ void __launch_bounds__(g_rows_per_cta<T>(), g_ctas_per_sm<T, PTS>())
   }
 }
 
+// ---- half rows ------------------------------------------------------------------
+// A forward sweep from zero needs only a row's entries in earlier colours, and
+// the residual after it (relax 1: (D + L) x = b holds then, see mc_up_residual)
+// is -U x over those in later colours.  Whether a neighbour's colour is earlier
+// depends on the row's colour and on the highest axis it is displaced along:
+//  27 points: displaced along axis 0 (planes 0..8, 18..26: group 4), else along
+//    axis 1 (9..11, 15..17: group 2), else along axis 2 (12, 14: group 1); the
+//    displacement flips that axis's colour bit, so the neighbour is earlier when
+//    the row's bit is set: the earlier groups are the bits of the colour c, the
+//    later ones those of ~c;
+//  7 points: every neighbour (group 1) has the other colour.
+// A launch reads only its groups' value planes: on average half of them.  The
+// sums run in offset order, so a sweep equals MODE 2's from zero bit for bit.
+// 256^3, whole rows / half rows: 27 points FP64 (FP64-pipe bound, half its FMAs)
+// 148 / 88 us per colour and 800 / 423 us for the residual; 7 points float 77 / 65
+// us for the second colour (whose residuals the whole row formed too) and 66 / 59
+// for the residual.  FP64 AMG-CG, 27 points, 501 -> 445 ms.
+template <int PTS>
+__host__ __device__ constexpr int g_group(int e) {
+  if (PTS == 7) return 1;
+  return g_dz<PTS>(e) != 0 ? 4 : g_dy<PTS>(e) != 0 ? 2 : 1;
+}
+template <int PTS, bool UP>
+__device__ __forceinline__ unsigned g_parts(int c) {
+  return (UP ? ~(unsigned)c : (unsigned)c) & (PTS == 27 ? 7u : 1u);
+}
+
+// x and value of entries [E0, E1) (one group, without the diagonal) into the
+// row, in rounds of kG27Batch whose loads go out together
+template <typename VT, typename XT, int PTS, int E0, int E1, class Row>
+__device__ __forceinline__ void g_run(const G27 &g, const GCell &cell, unsigned sides, int64_t r,
+                                      const VT *__restrict__ v, const XT *x, const G27Sor &so,
+                                      Row &row) {
+  constexpr int B = kG27Batch;
+#pragma unroll
+  for (int e0 = E0; e0 < E1; e0 += B) {
+    XT xv[B], av[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int e = e0 + u;
+      if (e >= E1) break;
+      av[u] = cvt<XT>(g27_ld(v + (int64_t)e * g.stride + r));
+      xv[u] = g27_ld(x + (g_in<PTS>(sides, e) ? g_nb<PTS>(g, cell, r, e) : r));
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const int e = e0 + u;
+      if (e >= E1) break;
+      row.step(e, g_in<PTS>(sides, e), av[u], xv[u], so);
+    }
+  }
+}
+
+// UP: y = -U x; else one colour of the sweep from zero, in place on x
+template <typename VT, typename XT, bool UP, int PTS>
+__global__ void __launch_bounds__(256)
+  k_g27_half(G27 g, int64_t rb, int64_t re, const VT *__restrict__ v, const XT *__restrict__ b,
+             XT *x, XT *__restrict__ y, G27Sor so) {
+  pdl_trigger();
+  pdl_wait();
+  const int64_t r = rb + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (r >= re) return;
+  const GCell cell = g_cell<PTS>(g, r);
+  const unsigned sides = g27_sides(g, cell.i, cell.j, cell.k);
+  const unsigned parts = g_parts<PTS, UP>(cell.c);
+  G27Row<VT, XT, UP ? 0 : 2, PTS> row;
+  if constexpr (!UP) {
+    row.init(r, b, x, so);
+    row.diag = cvt<XT>(g27_ld(v + (int64_t)g_diag<PTS>() * g.stride + r));
+  }
+  if constexpr (PTS == 27) {
+    if (parts & 4u) g_run<VT, XT, PTS, 0, 9>(g, cell, sides, r, v, (const XT *)x, so, row);
+    if (parts & 2u) g_run<VT, XT, PTS, 9, 12>(g, cell, sides, r, v, (const XT *)x, so, row);
+    if (parts & 1u) {
+      g_run<VT, XT, PTS, 12, 13>(g, cell, sides, r, v, (const XT *)x, so, row);
+      g_run<VT, XT, PTS, 14, 15>(g, cell, sides, r, v, (const XT *)x, so, row);
+    }
+    if (parts & 2u) g_run<VT, XT, PTS, 15, 18>(g, cell, sides, r, v, (const XT *)x, so, row);
+    if (parts & 4u) g_run<VT, XT, PTS, 18, 27>(g, cell, sides, r, v, (const XT *)x, so, row);
+  } else if (parts) {
+    g_run<VT, XT, PTS, 0, 3>(g, cell, sides, r, v, (const XT *)x, so, row);
+    g_run<VT, XT, PTS, 4, 7>(g, cell, sides, r, v, (const XT *)x, so, row);
+  }
+  if constexpr (UP) y[r] = -row.acc;
+  else row.finish(r, b, x, y, nullptr, so);
+}
+
+// The same on float rows with the value planes staged by the tensor engine as in
+// k_g27_vtma: boxes of 9, 3 and 1 planes of the groups that the tile's colours
+// need (7 points: the whole box of 7).
+struct GHalfMaps {
+  CUtensorMap m[3];  // boxes of 9, 3 and 1 planes (7 points: m[0] of 7)
+};
+
+template <bool UP, int PTS>
+__global__ void __launch_bounds__(256, PTS == 27 ? 4 : 6)
+  k_g27_vhalf(const __grid_constant__ GHalfMaps maps, G27 g, int64_t rb, int64_t re,
+              const float *__restrict__ b, float *x, float *__restrict__ y, G27Sor so, int *err) {
+  constexpr int RT = g_rows_per_cta<float>();
+  constexpr int kDiag = g_diag<PTS>();
+  __shared__ __align__(128) float sv[PTS * RT];
+  __shared__ uint64_t bar;
+  const int64_t t0 = rb + (int64_t)blockIdx.x * RT;
+  const int64_t t1 = min(t0 + RT, re) - 1;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned c0 = (unsigned)t0 / (unsigned)g.block, c1 = (unsigned)t1 / (unsigned)g.block;
+    const unsigned need = g_parts<PTS, UP>((int)c0) | g_parts<PTS, UP>((int)c1);
+    if constexpr (PTS == 27) {
+      const unsigned planes = (need & 4u ? 18u : 0u) + (need & 2u ? 6u : 0u) +
+                              (need & 1u ? 3u : UP ? 0u : 1u);
+      mbar_expect_tx(&bar, planes * RT * (unsigned)sizeof(float));
+      if (need & 4u) {
+        tma_load_2d(sv, &maps.m[0], (int)t0, 0, &bar);
+        tma_load_2d(sv + 18 * RT, &maps.m[0], (int)t0, 18, &bar);
+      }
+      if (need & 2u) {
+        tma_load_2d(sv + 9 * RT, &maps.m[1], (int)t0, 9, &bar);
+        tma_load_2d(sv + 15 * RT, &maps.m[1], (int)t0, 15, &bar);
+      }
+      if (need & 1u) tma_load_2d(sv + 12 * RT, &maps.m[1], (int)t0, 12, &bar);
+      else if (!UP) tma_load_2d(sv + 13 * RT, &maps.m[2], (int)t0, 13, &bar);
+    } else {
+      mbar_expect_tx(&bar, PTS * RT * (unsigned)sizeof(float));
+      tma_load_2d(sv, &maps.m[0], (int)t0, 0, &bar);
+    }
+  }
+  pdl_trigger();
+  pdl_wait();
+  const int64_t r = t0 + threadIdx.x;
+  const bool active = r < re;
+  G27Row<float, float, UP ? 0 : 2, PTS> row;
+  float xv[PTS];
+  unsigned sides = 0, parts = 0;
+  if (active) {
+    const GCell cell = g_cell<PTS>(g, r);
+    sides = g27_sides(g, cell.i, cell.j, cell.k);
+    parts = g_parts<PTS, UP>(cell.c);
+    if constexpr (!UP) row.init(r, b, x, so);
+#pragma unroll
+    for (int group = 4; group > 0; group >>= 1) {
+      if (!(parts & (unsigned)group)) continue;
+#pragma unroll
+      for (int e = 0; e < PTS; ++e)
+        if (e != kDiag && g_group<PTS>(e) == group)
+          xv[e] = g27_ld(x + (g_in<PTS>(sides, e) ? g_nb<PTS>(g, cell, r, e) : r));
+    }
+  }
+  if (!mbar_wait_bounded(&bar, 0)) {
+    // the copies did not complete in time: report, wait once more (bounded)
+    // for them and leave
+    if (threadIdx.x == 0) {
+      atomicExch(err, 1);
+      (void)mbar_wait_bounded(&bar, 0);
+    }
+    return;
+  }
+  if (!active) return;
+  const float *svt = sv + threadIdx.x;
+  auto run = [&](int e0, int e1, unsigned group) {
+    if (!(parts & group)) return;
+#pragma unroll
+    for (int e = 0; e < PTS; ++e)
+      if (e >= e0 && e < e1) row.step(e, g_in<PTS>(sides, e), svt[e * RT], xv[e], so);
+  };
+  if constexpr (!UP) row.diag = svt[kDiag * RT];
+  if constexpr (PTS == 27) {
+    run(0, 9, 4u);
+    run(9, 12, 2u);
+    run(12, 13, 1u);
+    run(14, 15, 1u);
+    run(15, 18, 2u);
+    run(18, 27, 4u);
+  } else {
+    run(0, 3, 1u);
+    run(4, 7, 1u);
+  }
+  if constexpr (UP) y[r] = -row.acc;
+  else row.finish(r, b, x, y, nullptr, so);
+}
+
 // the tensor-staged kernels serve float rows with 16-byte-aligned row starts
 // (LGX_G27_TMA=0 switches it off)
 static bool g27_tma_enabled() {
@@ -659,6 +847,57 @@ static const CUtensorMap *g27_value_map(const Grid27 &gr, const T *v) {
   return map;
 }
 
+// the boxes of k_g27_vhalf on the float values (null: no tensor maps)
+static bool g27_half_maps(const Grid27 &gr, const float *v, GHalfMaps *out) {
+  const G27EncodeFn encode = g27_encode();
+  if (!encode) return false;
+  const cuuint64_t gdim[2] = {(cuuint64_t)gr.stride, (cuuint64_t)gr.points};
+  const cuuint64_t gstride[1] = {(cuuint64_t)gr.stride * sizeof(float)};
+  const cuuint32_t estride[2] = {1, 1};
+  const int high[3] = {gr.points == 27 ? 9 : 7, 3, 1};
+  for (int k = 0; k < 3; ++k) {
+    const cuuint32_t box[2] = {(cuuint32_t)g_rows_per_cta<float>(), (cuuint32_t)high[k]};
+    if (encode(&out->m[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(v), gdim,
+               gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return false;
+  }
+  return true;
+}
+
+// one launch of the half rows [rb, re)
+template <typename VT, typename XT, bool UP, int PTS>
+static lgx_status launch_half_pts(const Grid27 &gr, const VT *v, int64_t rb, int64_t re,
+                                  const XT *b, XT *x, XT *y, const G27Sor &so, cudaStream_t s) {
+  const bool pdl = sizeof(XT) == 4 || re - rb <= pdl_fp64_rows();
+  if constexpr (std::is_same_v<VT, float> && std::is_same_v<XT, float>) {
+    GHalfMaps maps;
+    if (g27_tma_enabled() && rb % 4 == 0 && ((uintptr_t)v & 15u) == 0 &&
+        (gr.stride * (int64_t)sizeof(float)) % 16 == 0 && gr.stride <= (int64_t)INT32_MAX &&
+        g27_half_maps(gr, v, &maps)) {
+      constexpr int RT = g_rows_per_cta<float>();
+      LGX_CUDA(launch_pdl(pdl, k_g27_vhalf<UP, PTS>, dim3((unsigned)((re - rb + RT - 1) / RT)),
+                          dim3(RT), 0, s, maps, view(gr), rb, re, b, x, y, so,
+                          device_error_flag()));
+      count_launch();
+      return LGX_OK;
+    }
+  }
+  LGX_CUDA(launch_pdl(pdl, k_g27_half<VT, XT, UP, PTS>, dim3((unsigned)((re - rb + 255) / 256)),
+                      dim3(256), 0, s, view(gr), rb, re, v, b, x, y, so));
+  count_launch();
+  return LGX_OK;
+}
+
+template <typename VT, typename XT, bool UP>
+static lgx_status launch_half(const Grid27 &gr, const VT *v, int64_t rb, int64_t re, const XT *b,
+                              XT *x, XT *y, const G27Sor &so, cudaStream_t s) {
+  if (re <= rb) return LGX_OK;
+  if (gr.points == 7) return launch_half_pts<VT, XT, UP, 7>(gr, v, rb, re, b, x, y, so, s);
+  return launch_half_pts<VT, XT, UP, 27>(gr, v, rb, re, b, x, y, so, s);
+}
+
 template <typename T, int MODE, int PTS>
 static bool g27_tma_launch(const Grid27 &gr, const T *v, int64_t rb, int64_t re, const T *b, T *x,
                            T *y, const G27Sor &so, bool pdl, cudaStream_t s, lgx_status *st) {
@@ -671,7 +910,7 @@ static bool g27_tma_launch(const Grid27 &gr, const T *v, int64_t rb, int64_t re,
   constexpr int RT = g_rows_per_cta<T>();
   const int64_t ctas = (re - rb + RT - 1) / RT;
   auto kern = k_g27_vtma<T, MODE, false, PTS>;
-  if constexpr (g_sor_mode<MODE>())
+  if constexpr (MODE == 4)
     if (so.from_zero) kern = k_g27_vtma<T, MODE, true, PTS>;
   const cudaError_t e = launch_pdl(pdl, kern, dim3((unsigned)ctas), dim3(RT), 0, s, *map,
                                    view(gr), rb, re, b, x, y, so, device_error_flag());
@@ -801,6 +1040,13 @@ lgx_status grid_sor_rows(const Csr &a, const VT *val, int64_t rb, int64_t re, co
     }
   }
   if (r_out) return fail(LGX_ERR_UNSUPPORTED, "sweep with residual: FP64 or bfloat16 rows");
+  if constexpr (!kIsBf16<VT>) {
+    if (from_zero) {
+      LGX_CHECK((launch_half<VT, XT, false>(*a.grid, v, rb, re, b, x, nullptr, so, s)));
+      *done = true;
+      return LGX_OK;
+    }
+  }
   LGX_CHECK((launch_g27<VT, XT, 2>(*a.grid, v, rb, re, b, x, nullptr, scale, so, s)));
   *done = true;
   return LGX_OK;
@@ -815,6 +1061,20 @@ lgx_status grid_sor_rows(const Csr &a, const VT *val, int64_t rb, int64_t re, co
 // eighth of the residual pass at the price of a longer row, so it keeps the
 // pass.
 bool grid_sweep_residual(const Csr &a) { return a.grid && a.grid->points == 7; }
+
+template <typename VT, typename XT>
+lgx_status grid_up_residual(const Csr &a, const VT *val, const XT *x, XT *r, cudaStream_t s,
+                            bool *done) {
+  *done = false;
+  if (!a.grid) return LGX_OK;
+  const VT *v = grid_values(*a.grid, val);
+  if (!v) return LGX_OK;
+  // (the last colour's rows have no later colour: the restriction skips them)
+  LGX_CHECK((launch_half<VT, XT, true>(*a.grid, v, 0, a.n - a.grid->block, nullptr,
+                                       const_cast<XT *>(x), r, G27Sor{}, s)));
+  *done = true;
+  return LGX_OK;
+}
 
 template <typename VT, typename XT>
 lgx_status grid_residual_rows(const Csr &a, const VT *val, const XT *b, const XT *x, XT *r,
@@ -863,6 +1123,12 @@ template lgx_status grid_sor_rows<bf16, float>(const Csr &, const bf16 *, int64_
                                                const float *, float *, double, int,
                                                const double *, int, int, int64_t, const float *,
                                                cudaStream_t, bool *, float *);
+template lgx_status grid_up_residual<double, double>(const Csr &, const double *, const double *,
+                                                     double *, cudaStream_t, bool *);
+template lgx_status grid_up_residual<float, double>(const Csr &, const float *, const double *,
+                                                    double *, cudaStream_t, bool *);
+template lgx_status grid_up_residual<float, float>(const Csr &, const float *, const float *,
+                                                   float *, cudaStream_t, bool *);
 template lgx_status grid_residual_rows<double, double>(const Csr &, const double *,
                                                        const double *, const double *, double *,
                                                        int64_t, int64_t, cudaStream_t, bool *);

@@ -269,6 +269,11 @@ template <typename VT, typename XT>
 lgx_status grid_residual_rows(const Csr &a, const VT *val, const XT *b, const XT *x, XT *r,
                               int64_t rb, int64_t re, cudaStream_t s, bool *done);
 
+// -U x (mc_up_residual) of all rows but the last colour's
+template <typename VT, typename XT>
+lgx_status grid_up_residual(const Csr &a, const VT *val, const XT *x, XT *r, cudaStream_t s,
+                            bool *done);
+
 lgx_status stencil_spmv(const StencilDesc &st, const double *x, double *y, cudaStream_t s);
 lgx_status stencil_residual(const StencilDesc &st, const double *b, const double *x, double *r,
                             double *norm, double *partials, unsigned *counter, cudaStream_t s);
@@ -313,11 +318,14 @@ lgx_status colouring_make_bf16(lgx_colouring &c, cudaStream_t s);
 template <typename VT, typename XT>
 lgx_status mc_residual(const lgx_colouring &c, const VT *val, const XT *b, const XT *x, XT *r,
                        cudaStream_t s);
-// The residual of a natural-order level right after a forward sweep from zero
-// with relax 1 (not ultra): the sweep solved every row with its earlier
-// colours, (D + L) x = b, so what is left is -U x.
+// The residual right after a forward sweep from zero with relax 1 (not ultra):
+// the sweep solved every row with its earlier colours, (D + L) x = b, so what is
+// left is -U x.  Natural-order levels read their halves; levels in colour order
+// their grid rows or, from `val`, the entries of later colours, and leave the
+// last colour's rows (which are 0) unwritten.
 template <typename VT, typename XT>
-lgx_status mc_up_residual(const lgx_colouring &c, const XT *x, XT *r, cudaStream_t s);
+lgx_status mc_up_residual(const lgx_colouring &c, const VT *val, const XT *x, XT *r,
+                          cudaStream_t s);
 // gives c.pcsr a Grid27 when it is the parity-coloured 27-point (points 27)
 // or red-black 7-point (points 7) operator on `dims` (checked on the device;
 // *attached tells whether it was)

@@ -705,6 +705,35 @@ struct ListResidualOp {
   __device__ __forceinline__ void finish(double) const {}
 };
 
+// r = -U x on whole rows in colour order: row i's entries of later colours are
+// those right of i (no two rows of a colour are neighbours)
+template <typename VT, typename XT>
+struct LaterResidualOp {
+  const XT *x;
+  XT *r;
+  using X = XT;
+  static constexpr bool kReduce = false;
+  double *partials = nullptr;
+  unsigned *counter = nullptr;
+  template <int W, bool FLAT>
+  __device__ __forceinline__ double row(int64_t i, const int32_t *c, const VT *v, int len) const {
+    XT ax = XT(0);
+    for (int k = 0; k < len; k += W) {
+      int32_t cc[W];
+      XT xv[W];
+      row_columns<W>(c, k, len, cc);
+#pragma unroll
+      for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], k + u < len && cc[u] > i);
+#pragma unroll
+      for (int u = 0; u < W; ++u)
+        if (k + u < len && cc[u] > i) ax = fma(cvt<XT>(v[k + u]), xv[u], ax);
+    }
+    r[i] = -ax;
+    return 0.0;
+  }
+  __device__ __forceinline__ void finish(double) const {}
+};
+
 // First colour of a forward sweep from x = 0: every neighbour still reads 0,
 // so the row's products with them leave accum = b_i (an fma with a zero
 // product; where only the sign of a zero could differ, the row's result is
@@ -807,7 +836,15 @@ lgx_status mc_residual(const lgx_colouring &c, const VT *val, const XT *b, const
 }
 
 template <typename VT, typename XT>
-lgx_status mc_up_residual(const lgx_colouring &c, const XT *x, XT *r, cudaStream_t s) {
+lgx_status mc_up_residual(const lgx_colouring &c, const VT *val, const XT *x, XT *r,
+                          cudaStream_t s) {
+  if (!c.natural) {
+    bool done = false;
+    LGX_CHECK((grid_up_residual<VT, XT>(c.pcsr, val, x, r, s, &done)));
+    if (done || c.ncolours < 1) return LGX_OK;
+    return launch_rows<VT>(0, c.offsets[c.ncolours - 1], c.pcsr, val,
+                           LaterResidualOp<VT, XT>{x, r}, s);
+  }
   const VT *v;
   if constexpr (sizeof(VT) == 8) v = c.up.v64.p;
   else v = c.up.v32.p;
@@ -817,8 +854,8 @@ lgx_status mc_up_residual(const lgx_colouring &c, const XT *x, XT *r, cudaStream
 #define LGX_MC_RESIDUAL(VT, XT)                                                              \
   template lgx_status mc_residual<VT, XT>(const lgx_colouring &, const VT *, const XT *,     \
                                           const XT *, XT *, cudaStream_t);                   \
-  template lgx_status mc_up_residual<VT, XT>(const lgx_colouring &, const XT *, XT *,        \
-                                             cudaStream_t);
+  template lgx_status mc_up_residual<VT, XT>(const lgx_colouring &, const VT *, const XT *,  \
+                                             XT *, cudaStream_t);
 LGX_MC_RESIDUAL(double, double)
 LGX_MC_RESIDUAL(float, double)
 LGX_MC_RESIDUAL(float, float)

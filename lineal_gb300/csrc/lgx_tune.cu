@@ -233,13 +233,19 @@ lgx_status tune_level(lgx_colouring &c, const VT *val, const float *scale, doubl
       // the cycle's residual: the rows' later-colour halves (relax 1), or whole
       const bool up = relax == 1.0 && !ultra;
       LGX_CHECK(tune_slot((up ? c.up : p).tuned[0][vi], reps, s, e, [&](cudaStream_t cs) {
-        return up ? mc_up_residual<VT, XT>(c, v.x.p, v.r.p, cs)
+        return up ? mc_up_residual<VT, XT>(c, val, v.x.p, v.r.p, cs)
                   : mc_residual<VT, XT>(c, val, v.b.p, v.x.p, v.r.p, cs);
       }));
       set_slot(c, 0, vi, (int8_t)e.config);
     }
   }
-  if (!c.natural)
+  if constexpr (!kIsBf16<VT>) {
+    if (!c.natural && relax == 1.0 && !ultra)
+      LGX_CHECK(tune_slot(p.tuned[0][vi], reps, s, e, [&](cudaStream_t cs) {
+        return mc_up_residual<VT, XT>(c, val, v.x.p, v.r.p, cs);
+      }));
+  }
+  if (!c.natural && (kIsBf16<VT> || relax != 1.0 || ultra))
     LGX_CHECK(tune_slot(p.tuned[0][vi], reps, s, e, [&](cudaStream_t cs) {
       return csr_residual<VT, XT>(p, val, v.b.p, v.x.p, v.r.p, nullptr, nullptr, nullptr, cs,
                                   scale);
