@@ -246,6 +246,7 @@ struct AggDev {
   int64_t *pcount;      // aggregates per partition
   int64_t *stats;       // 5 counters (atomic adds)
   int32_t cap;          // k_aggregate_cta: front and connected-list capacity
+  int32_t cta_rows;     // k_aggregate_cta: row offsets in shared memory
 };
 
 __device__ __forceinline__ int64_t part_begin(int64_t n, int64_t p, int64_t k) {
@@ -611,10 +612,16 @@ __global__ void __launch_bounds__(32 * kAggWarpsPerBlock) k_aggregate(AggDev D) 
 //    warps 1.. wait between evaluations at a named barrier that warp 0
 //    releases;
 //  - choices are integer reductions (redux.sync) over 32-bit vertex ids
-//    and a 64-bit key.
+//    and the parts of the key, in registers for fronts of up to 32 members;
+//  - the lists are no longer than an aggregate's neighbours can be, the row
+//    offsets stand in shared memory where they fit, and the rest of the SM is
+//    left to the L1, which then holds the front's rows.
 // Measured at 256^3 against the warp kernel: levels 1-3 (174, 17, 8
 // partitions) 153 / 754 / 268 ms before, with 60 % of it evaluating fronts
-// of ~13 members one row per lane.  Decisions are the warp kernel's:
+// of ~13 members one row per lane.  The last two items, 998k rows, 27 points
+// (243, 10, 8, 6 partitions): 13.5 / 54.5 / 13.0 / 3.2 -> 8.8 / 38.4 / 9.2 /
+// 2.3 ms; of the second level's 112M cycles per partition the decisions took
+// 27M (now 7M), the vertices' rows 29M, the evaluations 28M.  Decisions are the warp kernel's:
 // counts are order-free sums, selections take the smallest vertex ids, a
 // member's position is found by search, and every aggregate's vertices are
 // added in the same order.  Capacities: local aggregate ids below 0xFFFE,
@@ -638,6 +645,11 @@ __host__ __device__ inline int64_t agg_cta_base(int64_t P) {
 }
 __host__ __device__ inline int64_t agg_cta_bytes(int64_t P, int64_t cap) {
   return agg_cta_base(P) + 30 * cap;
+}
+// the row offsets within the partition and the isolated bits, kept in shared
+// memory where the lists leave room for them
+__host__ __device__ inline int64_t agg_cta_rows_bytes(int64_t P) {
+  return agg_align16(4 * (P + 1)) + agg_align16(4 * agg_bit_words(P));
 }
 
 struct AggCtaCtl {
@@ -664,6 +676,9 @@ struct AggCta {
   int32_t *flen;    // per front position: row length, 0 for isolated members
   uint32_t *cntA, *cntB;  // per front position: packed 16-bit counts / mark
   uint16_t *conn;   // connected local aggregate ids
+  int32_t *srow = nullptr;   // by local vertex: row offset from ebase (or null)
+  uint32_t *sIso = nullptr;  // by local vertex: isolated
+  int64_t ebase = 0;
   // warp 0's state (warp-uniform)
   int64_t front_len = 0, conn_len = 0, counter = 0;
   int64_t st[5] = {0, 0, 0, 0, 0};
@@ -688,6 +703,35 @@ struct AggCta {
     cntB = cntA + cap;
     q += 16 * (int64_t)cap;
     conn = (uint16_t *)q;
+    if (D.cta_rows) {
+      q = smem + agg_align16(agg_cta_bytes(P, cap));
+      srow = (int32_t *)q;
+      sIso = (uint32_t *)(q + agg_align16(4 * (P + 1)));
+      ebase = D.rowptr[b];
+    }
+  }
+  // row of vertex v (in range) and whether it is isolated
+  __device__ void row_of(int64_t v, int64_t &rb, int64_t &re) const {
+    if (srow) {
+      rb = ebase + srow[v - pb];
+      re = ebase + srow[v - pb + 1];
+    } else {
+      rb = D.rowptr[v];
+      re = D.rowptr[v + 1];
+    }
+  }
+  __device__ bool iso_of(int64_t v) const {
+    if (!sIso) return D.iso[v];
+    const int64_t u = v - pb;
+    return (sIso[u >> 5] >> (u & 31)) & 1u;
+  }
+  // a new front member: its row on its way to the L1
+  __device__ void expect_row(int64_t v) const {
+    if (!srow) return;
+    const int64_t rb = ebase + srow[v - pb];
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(D.col + rb));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(D.dep + rb));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(D.inf + rb));
   }
   __device__ bool in_range(int64_t v) const { return v >= pb && v < pe; }
   __device__ int32_t &blen(uint32_t ag) const { return D.block_len[pb + ag]; }
@@ -823,12 +867,10 @@ struct AggCta {
           want_conn = ta < kIsolated && !connected(ta);
           want_front = ta == kUnaggregated && !in_front(t);
         }
-        const unsigned cmask = __ballot_sync(kFull, want_conn);
-        bool leader = false;
-        if (want_conn) {
-          const unsigned same = __match_any_sync(cmask, ta);
-          leader = (__ffs(same) - 1) == lane;
-        }
+        // one lane of each aggregate sets its bit and lists it (the list's order
+        // does not matter: it only says what to clear)
+        const bool leader =
+          want_conn && !((atomicOr(&cF[ta >> 5], 1u << (ta & 31)) >> (ta & 31)) & 1u);
         const unsigned lmask = __ballot_sync(kFull, leader);
         const unsigned fmask = __ballot_sync(kFull, want_front);
         if (conn_len + __popc(lmask) > cap || front_len + __popc(fmask) > cap) {
@@ -836,10 +878,7 @@ struct AggCta {
           return;
         }
         const unsigned below = (1u << lane) - 1u;
-        if (leader) {
-          conn[conn_len + __popc(lmask & below)] = (uint16_t)ta;
-          conn_flag(ta, true);
-        }
+        if (leader) conn[conn_len + __popc(lmask & below)] = (uint16_t)ta;
         conn_len += __popc(lmask);
         if (want_front) {
           front[front_len + __popc(fmask & below)] = (int32_t)t;
@@ -852,10 +891,12 @@ struct AggCta {
     bool long_row = false;
     for (int64_t q = f0 + lane; q < front_len; q += 32) {
       const int64_t t = front[q];
-      const int64_t rb = D.rowptr[t], re = D.rowptr[t + 1];
+      int64_t rb, re;
+      row_of(t, rb, re);
+      expect_row(t);
       fbeg[q] = rb;
       long_row = long_row || re - rb > 65535;
-      flen[q] = D.iso[t] ? 0 : (int32_t)(re - rb);
+      flen[q] = iso_of(t) ? 0 : (int32_t)(re - rb);
     }
     if (__any_sync(kFull, long_row)) bad = true;  // counts would not fit 16 bits
     __syncwarp();
@@ -873,7 +914,7 @@ struct AggCta {
       eb = ee = 0;
       return;
     }
-    const int64_t pos = pos1 - 1;
+    const int64_t pos = (int64_t)pos1 - 1;
     eb = fbeg[pos];
     ee = eb + flen[pos];
     __syncwarp();
@@ -889,11 +930,19 @@ struct AggCta {
   }
 
   __device__ void helpers_clear() {
-    for (int64_t i = lane; i < front_len; i += 32) front_flag(front[i], false);
-    for (int64_t i = lane; i < conn_len; i += 32) conn_flag(conn[i], false);
+    // (every set bit is listed, so whole words go)
+    for (int64_t i = lane; i < front_len; i += 32) inF[(front[i] - pb) >> 5] = 0u;
+    for (int64_t i = lane; i < conn_len; i += 32) cF[conn[i] >> 5] = 0u;
     front_len = 0;
     conn_len = 0;
     __syncwarp();
+  }
+
+  // floor(con 2^32 / den) for con <= den < 2^16, 2^32 - 1 for con == den
+  static __device__ uint32_t fraction(uint32_t con, uint32_t den) {
+    if (con == den) return 0xFFFFFFFFu;
+    const uint32_t q1 = (con << 16) / den, r1 = (con << 16) - q1 * den;
+    return q1 << 16 | (r1 << 16) / den;
   }
 
   // smallest member id > floor among the marked positions (mark in cntA);
@@ -909,17 +958,61 @@ struct AggCta {
 
   // grow_aggregate (base.hpp:532-585).  A member's key is (count,
   // connectivity, front neighbours) with connectivity = connected / (row
-  // length - 1) compared as doubles.  Here it is one 64-bit integer:
-  // count << 48 | floor(connected * (2^32 - 1) / (row length - 1)) << 16 |
-  // neighbours.  Distinct fractions with denominators below 2^16 differ by
-  // more than 1 / (2^32 - 1), so the scaled floors order and tie exactly as
-  // the fractions -- and as their correctly rounded quotients, which lie
-  // much closer than that apart only when equal.  Rows without a diagonal
-  // (a connected count above the denominator, or a zero denominator) are
-  // left to the warp kernel.
+  // length - 1) compared as doubles.  Here the fraction is floor(connected
+  // 2^32 / (row length - 1)): distinct fractions with denominators below 2^16
+  // differ by more than 2^-32, and the largest below 1 by more than 2^-16, so
+  // the scaled floors order and tie exactly as the fractions -- and as their
+  // correctly rounded quotients, which lie much closer than that apart only
+  // when equal.  Rows without a diagonal (a connected count above the
+  // denominator, or a zero denominator) are left to the warp kernel.  A front
+  // of up to 32 members is decided in registers, a member per lane, with one
+  // reduction per part of the key and the fractions only for members that tie
+  // in the count.
   __device__ void grow(uint32_t ag, int64_t &size) {
     while (size < D.min_size && front_len > 0) {
       eval(kCmdGrow, ag);
+      const int64_t room = D.max_size - size;
+      if (front_len <= 32) {
+        const bool on = lane < front_len;
+        const uint32_t ca = on ? cntA[lane] : 0u, cb = on ? cntB[lane] : 0u;
+        const uint32_t id = on ? (uint32_t)front[lane] : 0xFFFFFFFFu;
+        const uint32_t c = __any_sync(kFull, (ca & 0xFFFFu) != 0u) ? ca & 0xFFFFu : ca >> 16;
+        const uint32_t cmax = __reduce_max_sync(kFull, c);
+        if (cmax == 0) break;  // no candidates
+        bool cand = on && c == cmax;
+        unsigned m = __ballot_sync(kFull, cand);
+        if (m & (m - 1)) {
+          const uint32_t con = cb & 0xFFFFu, den = cand ? (uint32_t)flen[lane] - 1u : 1u;
+          if (__any_sync(kFull, cand && (den == 0u || con > den))) {
+            bad = true;
+            return;
+          }
+          // (every lane takes part in each reduction, candidates or not)
+          const uint32_t f = cand ? fraction(con, den) : 0u;
+          const uint32_t fmax = __reduce_max_sync(kFull, f);
+          cand = cand && f == fmax;
+          const uint32_t nb = cand ? (cb >> 16) + 1u : 0u;
+          const uint32_t nbmax = __reduce_max_sync(kFull, nb);
+          cand = cand && nb == nbmax;
+          m = __ballot_sync(kFull, cand);
+        }
+        if (m == 0u) {  // (a maximum always has its lane; guarded all the same)
+          bad = true;
+          return;
+        }
+        const int npick = (int)(__popc(m) < room ? __popc(m) : room);
+        uint32_t mine = cand ? id : 0xFFFFFFFFu;  // (survives the front's changes)
+        for (int k = 0; k < npick; ++k) {
+          const uint32_t v = __reduce_min_sync(kFull, mine);
+          if (mine == v) mine = 0xFFFFFFFFu;
+          int64_t eb, ee;
+          front_take(v, eb, ee);
+          if (bad) return;
+          add_help(v, ag, size, eb, ee);
+          if (bad) return;
+        }
+        continue;
+      }
       bool any2 = false;
       for (int64_t i = lane; i < front_len; i += 32) any2 = any2 || (cntA[i] & 0xFFFFu) != 0;
       const bool mode2 = __any_sync(kFull, any2);
@@ -929,12 +1022,12 @@ struct AggCta {
         const uint32_t c = mode2 ? cntA[i] & 0xFFFFu : cntA[i] >> 16;
         uint64_t key = 0;
         if (c > 0) {
-          const uint64_t con = cntB[i] & 0xFFFFu, nb = cntB[i] >> 16;
-          const uint64_t den = (uint64_t)(flen[i] - 1);
+          const uint32_t con = cntB[i] & 0xFFFFu, nb = cntB[i] >> 16;
+          const uint32_t den = (uint32_t)flen[i] - 1u;
           if (den == 0 || con > den) {
             odd = true;
           } else {
-            key = (uint64_t)c << 48 | (con * 0xFFFFFFFFull / den) << 16 | nb;
+            key = (uint64_t)c << 48 | (uint64_t)fraction(con, den) << 16 | nb;
           }
         }
         cntA[i] = (uint32_t)(key >> 32);
@@ -961,7 +1054,6 @@ struct AggCta {
         nmarked += __popc(__ballot_sync(kFull, m));
       }
       __syncwarp();
-      const int64_t room = D.max_size - size;
       const int64_t npick = nmarked < room ? nmarked : room;
       uint32_t picked[64];
       uint32_t floor = 0xFFFFFFFFu;
@@ -1002,8 +1094,9 @@ struct AggCta {
   // handle_vertex (base.hpp:638-677)
   __device__ void handle(int64_t seed) {
     if (agg_of(seed) != kUnaggregated) return;
-    const bool iso = D.iso[seed];
-    const int64_t eb = D.rowptr[seed], ee = D.rowptr[seed + 1];
+    const bool iso = iso_of(seed);
+    int64_t eb, ee;
+    row_of(seed, eb, ee);
     if (iso) {
       if (lane == 0) set_agg(seed, kIsolated);
       __syncwarp();
@@ -1083,6 +1176,16 @@ __global__ void __launch_bounds__(kAggCtaThreads) k_aggregate_cta(AggDev D, int 
     D.block_len[pb + u] = 0;
   }
   for (int64_t w = threadIdx.x; w < 2 * agg_bit_words(P); w += kAggCtaThreads) S.inF[w] = 0u;
+  if (S.srow) {
+    for (int64_t u = threadIdx.x; u <= P; u += kAggCtaThreads)
+      S.srow[u] = (int32_t)(D.rowptr[pb + u] - S.ebase);
+    for (int64_t w = threadIdx.x; w < agg_bit_words(P); w += kAggCtaThreads) {
+      uint32_t bits = 0u;
+      for (int64_t u = 32 * w; u < 32 * w + 32 && u < P; ++u)
+        bits |= (uint32_t)(D.iso[pb + u] != 0) << (u & 31);
+      S.sIso[w] = bits;
+    }
+  }
   if (threadIdx.x == 0) {
     ctl.cmd = kCmdGrow;
     ctl.bad = 0;
@@ -1181,14 +1284,23 @@ __global__ void k_agg_lists(AggDev D, const int64_t *poff, int64_t nc, const int
 // Capacity of the CTA kernel's lists for a level, 0 where it does not fit:
 // the shared memory of an SM is shared by the partitions it must hold at
 // once (1 KB of it reserved per CTA).
-static int32_t agg_cta_cap(int64_t n, int64_t nparts, int64_t smem_optin, int64_t smem_sm,
-                           int64_t sms, bool forced) {
+static int32_t agg_cta_cap(int64_t n, int64_t nnz, int64_t most, int64_t nparts,
+                           int64_t smem_optin, int64_t smem_sm, int64_t sms, bool forced,
+                           bool *rows) {
+  *rows = false;
   const int64_t pmax = (n + nparts - 1) / nparts;
   const int64_t per_sm = (nparts + sms - 1) / sms;
   const int64_t budget =
     std::min<int64_t>(smem_optin, smem_sm / per_sm - 1024 - (int64_t)sizeof(AggCtaCtl));
   const int64_t avail = budget - agg_cta_base(pmax) - 16;
-  int64_t cap = std::min<int64_t>(kAggCtaCapMax, avail > 0 ? avail / 30 / 8 * 8 : 0);
+  // an aggregate's vertices have at most `most` neighbours: longer lists would
+  // only take room from the L1, which holds the front's rows
+  const int64_t enough = std::max<int64_t>((most + 7) / 8 * 8, kAggCtaCapMin);
+  int64_t cap = std::min<int64_t>({(int64_t)kAggCtaCapMax, enough,
+                                   avail > 0 ? avail / 30 / 8 * 8 : (int64_t)0});
+  // (row offsets within a partition are 32-bit)
+  const int64_t left = avail - agg_cta_rows_bytes(pmax) - 16;
+  *rows = nnz <= (int64_t)INT32_MAX && left >= 30 * cap;
   if (const char *e = std::getenv("LGX_AGG_CTA_CAP")) {
     const long v = std::strtol(e, nullptr, 10);
     if (v >= 8) cap = std::min<int64_t>(cap, v / 8 * 8);
@@ -1220,8 +1332,11 @@ lgx_status aggregate(const Csr &a, const uint8_t *dep, const uint8_t *inf, const
   const char *force = std::getenv("LGX_AGG_KERNEL");
   const bool want_warp = force && std::strcmp(force, "warp") == 0;
   const bool forced_cta = force && std::strcmp(force, "cta") == 0;
+  bool rows = false;
   const int32_t cap =
-    n > 0 && !want_warp ? agg_cta_cap(n, nparts, smem_optin, smem_sm, sms, forced_cta) : 0;
+    n > 0 && !want_warp
+      ? agg_cta_cap(n, a.nnz, max_size * a.max_row, nparts, smem_optin, smem_sm, sms, forced_cta, &rows)
+      : 0;
   DBuf<int32_t> front, front_pos, conn, blocks, blen, eval;
   DBuf<uint8_t> conn_flag;
   DBuf<int64_t> pcount, poff, stats, glen;
@@ -1234,15 +1349,22 @@ lgx_status aggregate(const Csr &a, const uint8_t *dep, const uint8_t *inf, const
   LGX_CUDA(cudaMemsetAsync(pcount.p, 0, sizeof(int64_t) * nparts, s));
   AggDev D{a.rowptr.p, a.col.p,  dep,      inf,        iso,     agg,    n,
            nparts,     min_size, max_size, aggressive, nullptr, nullptr, nullptr,
-           nullptr,    blocks.p, blen.p,   nullptr,    pcount.p, stats.p, cap};
+           nullptr,    blocks.p, blen.p,   nullptr,    pcount.p, stats.p, cap, rows};
   bool done = n == 0;
   if (cap > 0) {
-    const int bytes = (int)agg_cta_bytes((n + nparts - 1) / nparts, cap);
+    const int64_t pmax = (n + nparts - 1) / nparts;
+    const int bytes = (int)(agg_align16(agg_cta_bytes(pmax, cap)) +
+                            (rows ? agg_cta_rows_bytes(pmax) : 0));
     DBuf<int> overflow;
     LGX_CHECK(overflow.alloc(1));
     LGX_CUDA(cudaMemsetAsync(overflow.p, 0, sizeof(int), s));
     LGX_CUDA(cudaFuncSetAttribute(k_aggregate_cta, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   bytes));
+    // no more of the SM for shared memory than its CTAs use: the rest is L1
+    const int64_t per_sm = (nparts + sms - 1) / sms;
+    const int64_t used = per_sm * (bytes + 1024 + (int64_t)sizeof(AggCtaCtl));
+    LGX_CUDA(cudaFuncSetAttribute(k_aggregate_cta, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)std::min<int64_t>(100, (used * 100 + smem_sm - 1) / smem_sm)));
     k_aggregate_cta<<<(unsigned)nparts, kAggCtaThreads, bytes, s>>>(D, overflow.p);
     LGX_LAUNCH_CHECK();
     int of = 0;
