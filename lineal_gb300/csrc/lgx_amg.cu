@@ -1867,8 +1867,74 @@ __device__ bool bchol_diag(double (*D)[kCb + 1], int nb) {
   return ok;
 }
 
-__global__ void __launch_bounds__(256) k_bchol_panel(int64_t n, int64_t k0, double *a, int *bad) {
-  __shared__ double D[kCb][kCb + 1];
+// The same factorisation (each entry's operations in the same order) by the 256
+// threads of a CTA: warp 0 takes the pivot's root and scales its column, then
+// thread t updates the entries t & 7, + 8, + 16, + 24 of row t >> 3.  One warp
+// walking each row's update in turn took two thirds of the 140 us of a panel.
+__device__ bool bchol_diag_cta(double (*D)[kCb + 1], int nb) {
+  const int t = threadIdx.x, r = t >> 3, c0 = t & 7;
+  bool ok = true;
+  for (int j = 0; j < nb; ++j) {
+    if (t < 32) {
+      const double d = D[j][j];
+      if (!(d > 0.0) || !isfinite(d)) ok = false;
+      const double ljj = sqrt(d);
+      __syncwarp();
+      if (t == j) D[j][j] = ljj;
+      if (t > j && t < nb) D[t][j] = D[t][j] / ljj;
+    }
+    __syncthreads();
+    if (r > j && r < nb) {
+      const double l = D[r][j];
+#pragma unroll
+      for (int q = 0; q < kCb / 8; ++q) {
+        const int c = c0 + 8 * q;
+        if (c > j && c <= r) D[r][c] = fma(-l, D[c][j], D[r][c]);
+      }
+    }
+    __syncthreads();
+  }
+  return ok;
+}
+
+// x L^T = s (a row below the panel) or L x = s (a column of the inverse's panel)
+// for a lower triangle in shared memory, four lanes per system: lane q holds the
+// entries q, q + 4, ... in s.  Per entry the operations of the plain substitution
+// in its order, the quotients through reciprocals (dinv: correctly rounded, 0
+// where the quotient divides; div_by_recip: the same bits).  A thread per system
+// left the panel's rows to n / 256 CTAs, each warp 500 FP64 FMAs long.
+__device__ __forceinline__ void tri_solve4(const double (*D)[kCb + 1], const double *dinv, int nb,
+                                           double (&s)[kCb / 4]) {
+  const int lane = threadIdx.x & 31, q = lane & 3, g0 = lane & ~3;
+#pragma unroll
+  for (int j = 0; j < kCb; ++j) {
+    if (j >= nb) break;
+    const int k = j >> 2, owner = j & 3;
+    double v = s[k];
+    if (q == owner) {
+      const double y = dinv[j];
+      // (a zero stays as it is: the pivots are positive)
+      if (nonzero_bits(v))
+        v = nonzero_bits(y) && exponent_within_400(v) ? div_by_recip(v, D[j][j], y) : v / D[j][j];
+      s[k] = v;
+    }
+    const double x = __shfl_sync(0xffffffffu, v, g0 + owner);
+    if (q > owner && 4 * k + q < nb) s[k] = fma(-x, D[4 * k + q][j], s[k]);
+#pragma unroll
+    for (int m = k + 1; m < kCb / 4; ++m)
+      if (4 * m + q < nb) s[m] = fma(-x, D[4 * m + q][j], s[m]);
+  }
+}
+
+__device__ __forceinline__ double pivot_recip(double d) {
+  return exponent_within_400(d) ? 1.0 / d : 0.0;
+}
+
+// (With several CTAs, CTA 0 leaves L_KK in lkk for k_bchol_trail to store: a CTA
+// that starts late still has to read A_KK.)
+__global__ void __launch_bounds__(256) k_bchol_panel(int64_t n, int64_t k0, double *a, double *lkk,
+                                                     int *bad) {
+  __shared__ double D[kCb][kCb + 1], dinv[kCb];
   if (*bad) return;
   const int nb = (int)(n - k0 < kCb ? n - k0 : kCb);
   const int64_t k1 = k0 + nb;
@@ -1877,43 +1943,42 @@ __global__ void __launch_bounds__(256) k_bchol_panel(int64_t n, int64_t k0, doub
     D[r][c] = c <= r ? a[(k0 + r) * n + k0 + c] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const bool ok = bchol_diag(D, nb);
-    if (!ok && threadIdx.x == 0) atomicOr(bad, 1);
-  }
+  const bool ok = bchol_diag_cta(D, nb);
+  if (threadIdx.x == 0 && !ok) atomicOr(bad, 1);
+  if (threadIdx.x < nb) dinv[threadIdx.x] = pivot_recip(D[threadIdx.x][threadIdx.x]);
   __syncthreads();
   if (blockIdx.x == 0)
     for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
       const int r = t / nb, c = t % nb;
-      if (c <= r) a[(k0 + r) * n + k0 + c] = D[r][c];
+      if (c <= r) *(gridDim.x > 1 ? lkk + r * kCb + c : a + (k0 + r) * n + k0 + c) = D[r][c];
     }
   // rows below the panel: x_j = (a_j - sum_{m<j} x_m l_jm) / l_jj
-  const int64_t i = k1 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double x[kCb];
-  double *row = a + i * n + k0;
+  const int q = threadIdx.x & 3;
+  const int64_t i = k1 + ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 4;
+  const bool on = i < n;
+  double *row = a + (on ? i : n - 1) * n + k0;
+  double s[kCb / 4];
 #pragma unroll
-  for (int j = 0; j < kCb; ++j) x[j] = j < nb ? row[j] : 0.0;
+  for (int k = 0; k < kCb / 4; ++k) s[k] = on && 4 * k + q < nb ? row[4 * k + q] : 0.0;
+  tri_solve4(D, dinv, nb, s);
 #pragma unroll
-  for (int j = 0; j < kCb; ++j) {
-    if (j >= nb) break;
-    double s = x[j];
-#pragma unroll
-    for (int m = 0; m < j; ++m) s = fma(-x[m], D[j][m], s);
-    x[j] = s / D[j][j];
-  }
-#pragma unroll
-  for (int j = 0; j < kCb; ++j)
-    if (j < nb) row[j] = x[j];
+  for (int k = 0; k < kCb / 4; ++k)
+    if (on && 4 * k + q < nb) row[4 * k + q] = s[k];
 }
 
 // lower tiles (I >= J) of the trailing matrix rows/columns >= k1
+// (and, where the panel had several CTAs, L_KK)
 __global__ void __launch_bounds__(256) k_bchol_trail(int64_t n, int64_t k0, double *a,
-                                                     const int *bad) {
+                                                     const double *lkk, const int *bad) {
   __shared__ double LI[32][kCb + 1], LJ[32][kCb + 1];
   if (*bad) return;
   const int nb = (int)(n - k0 < kCb ? n - k0 : kCb);
   const int64_t k1 = k0 + nb;
+  if (lkk && blockIdx.x == 0)
+    for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
+      const int r = t / nb, c = t % nb;
+      if (c <= r) a[(k0 + r) * n + k0 + c] = lkk[r * kCb + c];
+    }
   // tile t -> (I, J) with J <= I, row-major over the lower triangle
   const int64_t t = blockIdx.x;
   int64_t I = (int64_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
@@ -1947,33 +2012,30 @@ __global__ void __launch_bounds__(256) k_bchol_trail(int64_t n, int64_t k0, doub
     }
 }
 
-// X_KC = L_KK^-1 X_KC for the columns c < k1, one column per thread
+// X_KC = L_KK^-1 X_KC for the columns c < k1, four lanes per column
 __global__ void __launch_bounds__(256) k_btri_diag(int64_t n, int64_t k0, const double *l,
                                                    double *x) {
-  __shared__ double D[kCb][kCb + 1];
+  __shared__ double D[kCb][kCb + 1], dinv[kCb];
   const int nb = (int)(n - k0 < kCb ? n - k0 : kCb);
   const int64_t k1 = k0 + nb;
   for (int t = threadIdx.x; t < nb * nb; t += blockDim.x) {
     const int r = t / nb, c = t % nb;
-    D[r][c] = c <= r ? l[(k0 + r) * n + k0 + c] : 0.0;
+    const double v = c <= r ? l[(k0 + r) * n + k0 + c] : 0.0;
+    D[r][c] = v;
+    if (r == c) dinv[r] = pivot_recip(v);
   }
   __syncthreads();
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= k1) return;
-  double y[kCb];
+  const int q = threadIdx.x & 3;
+  const int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 4;
+  const bool on = c < k1;
+  double y[kCb / 4];
 #pragma unroll
-  for (int j = 0; j < kCb; ++j) y[j] = j < nb ? x[(k0 + j) * n + c] : 0.0;
+  for (int k = 0; k < kCb / 4; ++k)
+    y[k] = on && 4 * k + q < nb ? x[(k0 + 4 * k + q) * n + c] : 0.0;
+  tri_solve4(D, dinv, nb, y);
 #pragma unroll
-  for (int j = 0; j < kCb; ++j) {
-    if (j >= nb) break;
-    double s = y[j];
-#pragma unroll
-    for (int m = 0; m < j; ++m) s = fma(-D[j][m], y[m], s);
-    y[j] = s / D[j][j];
-  }
-#pragma unroll
-  for (int j = 0; j < kCb; ++j)
-    if (j < nb) x[(k0 + j) * n + c] = y[j];
+  for (int k = 0; k < kCb / 4; ++k)
+    if (on && 4 * k + q < nb) x[(k0 + 4 * k + q) * n + c] = y[k];
 }
 
 // X_IC -= L_IK X_KC for the rows i >= k1 and the columns c < k1 (32 x 32
@@ -2301,13 +2363,16 @@ lgx_status dense_inverse(const Csr &a, cudaStream_t s, DBuf<double> &inv, int sp
     }();
     if (blocked) {
       const int64_t npan = (n + kCb - 1) / kCb;
+      DBuf<double> lkk;
+      LGX_CHECK(lkk.alloc(kCb * kCb));
       for (int64_t K = 0; K < npan; ++K) {
         const int64_t k0 = K * kCb, k1 = std::min<int64_t>(k0 + kCb, n), below = n - k1;
-        k_bchol_panel<<<(unsigned)std::max<int64_t>(1, (below + 255) / 256), 256, 0, s>>>(
-          n, k0, l.p, bad.p);
+        const int64_t ctas = std::max<int64_t>(1, (4 * below + 255) / 256);
+        k_bchol_panel<<<(unsigned)ctas, 256, 0, s>>>(n, k0, l.p, lkk.p, bad.p);
         if (below > 0) {
           const int64_t T = (below + 31) / 32;
-          k_bchol_trail<<<(unsigned)(T * (T + 1) / 2), 256, 0, s>>>(n, k0, l.p, bad.p);
+          k_bchol_trail<<<(unsigned)(T * (T + 1) / 2), 256, 0, s>>>(
+            n, k0, l.p, ctas > 1 ? lkk.p : nullptr, bad.p);
         }
       }
       LGX_LAUNCH_CHECK();
@@ -2321,7 +2386,7 @@ lgx_status dense_inverse(const Csr &a, cudaStream_t s, DBuf<double> &inv, int sp
         n, xl.p);
       for (int64_t K = 0; K < npan; ++K) {
         const int64_t k0 = K * kCb, k1 = std::min<int64_t>(k0 + kCb, n), below = n - k1;
-        k_btri_diag<<<(unsigned)((k1 + 255) / 256), 256, 0, s>>>(n, k0, l.p, xl.p);
+        k_btri_diag<<<(unsigned)((4 * k1 + 255) / 256), 256, 0, s>>>(n, k0, l.p, xl.p);
         if (below > 0)
           k_btri_update<<<dim3((unsigned)((below + 31) / 32), (unsigned)((k1 + 31) / 32)), 256, 0,
                           s>>>(n, k0, l.p, xl.p);
