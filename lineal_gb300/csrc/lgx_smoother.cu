@@ -118,17 +118,44 @@ __global__ void k_jp_round(int64_t n, const int64_t *__restrict__ rowptr,
   }
 }
 
-__global__ void k_jp_commit(int64_t n, int32_t *colour, const int32_t *next,
-                            unsigned long long *remaining, int *maxc) {
+// the round's colours, the vertices still without one and the highest colour
+// (one atomic per block: one per vertex on a single address serialised a round)
+__global__ void __launch_bounds__(256) k_jp_commit(int64_t n, int32_t *colour,
+                                                   const int32_t *next,
+                                                   unsigned long long *remaining, int *maxc) {
+  __shared__ int part[2][8];
+  int left = 0, top = -1;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    if (next[i] >= 0) {
-      colour[i] = next[i];
-      atomicMax(maxc, next[i]);
+    const int32_t c = next[i];
+    if (c >= 0) {
+      colour[i] = c;
+      top = max(top, c);
+    } else {
+      left += colour[i] < 0;
     }
-    if (colour[i] < 0) atomicAdd(remaining, 1ull);
+  }
+  left = __reduce_add_sync(0xffffffffu, left);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = left;
+    part[1][threadIdx.x >> 5] = top;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      left += part[0][w];
+      top = max(top, part[1][w]);
+    }
+    if (left) atomicAdd(remaining, (unsigned long long)left);
+    if (top >= 0) atomicMax(maxc, top);
   }
 }
+
+// rounds launched between two looks at what remains: a round with nothing left
+// changes nothing, and a look costs the host about 20 us.  170k rows: 3.8 -> 2.4 ms
+// with the order below
+constexpr int kJpRounds = 4;
 
 lgx_status colouring_jp(const Csr &a, uint64_t seed, cudaStream_t s, DBuf<int32_t> &colour,
                         int32_t &ncolours) {
@@ -146,12 +173,16 @@ lgx_status colouring_jp(const Csr &a, uint64_t seed, cudaStream_t s, DBuf<int32_
   unsigned long long h_rem = (unsigned long long)n;
   int64_t rounds = 0;
   while (h_rem > 0) {
-    if (++rounds > n + 1) return fail(LGX_ERR_INVALID, "colouring did not terminate");
-    k_jp_round<<<g, 256, 0, s>>>(n, a.rowptr.p, a.col.p, seed, colour.p, next.p);
-    LGX_LAUNCH_CHECK();
-    LGX_CUDA(cudaMemsetAsync(rem.p, 0, sizeof(unsigned long long), s));
-    k_jp_commit<<<g, 256, 0, s>>>(n, colour.p, next.p, rem.p, maxc.p);
-    LGX_LAUNCH_CHECK();
+    if ((rounds += kJpRounds) > n + kJpRounds)
+      return fail(LGX_ERR_INVALID, "colouring did not terminate");
+    for (int q = 0; q < kJpRounds; ++q) {
+      k_jp_round<<<g, 256, 0, s>>>(n, a.rowptr.p, a.col.p, seed, colour.p, next.p);
+      LGX_LAUNCH_CHECK();
+      if (q == kJpRounds - 1)
+        LGX_CUDA(cudaMemsetAsync(rem.p, 0, sizeof(unsigned long long), s));
+      k_jp_commit<<<g, 256, 0, s>>>(n, colour.p, next.p, rem.p, maxc.p);
+      LGX_LAUNCH_CHECK();
+    }
     LGX_CUDA(cudaMemcpyAsync(&h_rem, rem.p, sizeof(h_rem), cudaMemcpyDeviceToHost, s));
     LGX_CUDA(cudaStreamSynchronize(s));
   }
@@ -180,6 +211,63 @@ __global__ void k_colour_place(int64_t n, const int32_t *colour, int32_t c, cons
     const int64_t p = base + pos[i];
     perm[p] = (int32_t)i;
     iperm[i] = (int32_t)p;
+  }
+}
+
+// The row order of up to kSortColours colours as one stable counting sort: rows
+// in blocks of kSortRows, counts per colour and block (table[c * blocks + block]),
+// their prefix sums, placement.  Bound by latency (three launches and a prefix sum);
+// a flag, a scan and a placement per colour with a host round trip each took, with
+// the rounds of the colouring before it, 2.4 ms on a level of 32k rows and 16
+// colours, now 1.65.  More colours than a block's counters hold keep the passes.
+constexpr int kSortColours = 64, kSortRows = 1024;
+
+__global__ void __launch_bounds__(256) k_colour_count(int64_t n, const int32_t *__restrict__ colour,
+                                                      int32_t ncolours, int64_t blocks,
+                                                      int64_t *__restrict__ table, int *bad) {
+  __shared__ int count[kSortColours];
+  if (threadIdx.x < kSortColours) count[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t i0 = (int64_t)blockIdx.x * kSortRows;
+  for (int64_t i = i0 + threadIdx.x; i < i0 + kSortRows && i < n; i += 256) {
+    const int32_t c = colour[i];
+    if (c < 0 || c >= ncolours) atomicOr(bad, 1);
+    else atomicAdd(&count[c], 1);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < ncolours) table[threadIdx.x * blocks + blockIdx.x] = count[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(256) k_colour_sort(int64_t n, const int32_t *__restrict__ colour,
+                                                     int32_t ncolours, int64_t blocks,
+                                                     const int64_t *__restrict__ start,
+                                                     int32_t *__restrict__ perm,
+                                                     int32_t *__restrict__ iperm) {
+  __shared__ int64_t at[kSortColours];
+  __shared__ int count[8][kSortColours];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if ((int)threadIdx.x < ncolours) at[threadIdx.x] = start[threadIdx.x * blocks + blockIdx.x];
+  const int64_t i0 = (int64_t)blockIdx.x * kSortRows;
+  for (int64_t base = i0; base < i0 + kSortRows && base < n; base += 256) {
+    for (int k = threadIdx.x; k < 8 * kSortColours; k += 256) (&count[0][0])[k] = 0;
+    __syncthreads();
+    const int64_t i = base + threadIdx.x;
+    int32_t c = i < n ? colour[i] : -1;
+    if (c >= ncolours) c = -1;
+    const unsigned same = __match_any_sync(0xffffffffu, c);
+    const int rank = __popc(same & ((1u << lane) - 1));
+    if (c >= 0 && rank == 0) count[w][c] = __popc(same);
+    __syncthreads();
+    if (c >= 0) {
+      int64_t p = at[c] + rank;
+      for (int v = 0; v < w; ++v) p += count[v][c];
+      perm[p] = (int32_t)i;
+      iperm[i] = (int32_t)p;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < ncolours)
+      for (int v = 0; v < 8; ++v) at[threadIdx.x] += count[v][threadIdx.x];
+    __syncthreads();
   }
 }
 
@@ -262,23 +350,43 @@ static lgx_status colouring_order(const Csr &a, const int32_t *d_colour, int32_t
   DBuf<int64_t> pos;
   DBuf<int> bad;
   LGX_CHECK(flag.alloc(n));
-  LGX_CHECK(pos.alloc(n + 1));
   LGX_CHECK(bad.alloc(1));
   LGX_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
   const unsigned g = (unsigned)std::min<int64_t>(grid_for(n, 256), 16384);
   out.offsets.assign((size_t)ncolours + 1, 0);
   int64_t base = 0;
-  for (int32_t c = 0; c < ncolours; ++c) {
-    k_colour_flag<<<g, 256, 0, s>>>(n, out.colour.p, c, flag.p, bad.p, ncolours);
+  if (n > 0 && ncolours <= kSortColours) {
+    const int64_t blocks = (n + kSortRows - 1) / kSortRows, entries = ncolours * blocks;
+    DBuf<int64_t> table;
+    LGX_CHECK(table.alloc(entries));
+    LGX_CHECK(pos.alloc(entries + 1));
+    k_colour_count<<<(unsigned)blocks, 256, 0, s>>>(n, out.colour.p, ncolours, blocks, table.p,
+                                                    bad.p);
     LGX_LAUNCH_CHECK();
-    LGX_CHECK(inclusive_offsets(n, flag.p, pos.p, s));
-    k_colour_place<<<g, 256, 0, s>>>(n, out.colour.p, c, pos.p, base, out.perm.p, out.iperm.p);
+    LGX_CHECK(inclusive_offsets(entries, table.p, pos.p, s));
+    k_colour_sort<<<(unsigned)blocks, 256, 0, s>>>(n, out.colour.p, ncolours, blocks, pos.p,
+                                                   out.perm.p, out.iperm.p);
     LGX_LAUNCH_CHECK();
-    int64_t cnt = 0;
-    LGX_CUDA(cudaMemcpyAsync(&cnt, pos.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    // the colours' first entries of the prefix sums, and the total
+    LGX_CUDA(cudaMemcpy2DAsync(out.offsets.data(), sizeof(int64_t), pos.p,
+                               sizeof(int64_t) * (size_t)blocks, sizeof(int64_t),
+                               (size_t)ncolours, cudaMemcpyDeviceToHost, s));
+    LGX_CUDA(cudaMemcpyAsync(&base, pos.p + entries, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     LGX_CUDA(cudaStreamSynchronize(s));
-    out.offsets[c] = base;
-    base += cnt;
+  } else {
+    LGX_CHECK(pos.alloc(n + 1));
+    for (int32_t c = 0; c < ncolours; ++c) {
+      k_colour_flag<<<g, 256, 0, s>>>(n, out.colour.p, c, flag.p, bad.p, ncolours);
+      LGX_LAUNCH_CHECK();
+      LGX_CHECK(inclusive_offsets(n, flag.p, pos.p, s));
+      k_colour_place<<<g, 256, 0, s>>>(n, out.colour.p, c, pos.p, base, out.perm.p, out.iperm.p);
+      LGX_LAUNCH_CHECK();
+      int64_t cnt = 0;
+      LGX_CUDA(cudaMemcpyAsync(&cnt, pos.p + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      LGX_CUDA(cudaStreamSynchronize(s));
+      out.offsets[c] = base;
+      base += cnt;
+    }
   }
   out.offsets[ncolours] = base;
   k_colour_validate<<<g, 256, 0, s>>>(n, a.rowptr.p, a.col.p, out.colour.p, bad.p);
