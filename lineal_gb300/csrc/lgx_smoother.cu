@@ -72,122 +72,145 @@ __device__ __forceinline__ uint64_t splitmix(uint64_t seed, uint64_t i) {
   return z ^ (z >> 31);
 }
 
-// One Jones-Plassmann round (see the oracle's lo_colour_jp): a vertex that
-// beats all uncoloured neighbours on (priority, index) takes the smallest
-// colour unused by coloured neighbours.  Colours of this round go to `next`.
-__global__ void k_jp_round(int64_t n, const int64_t *__restrict__ rowptr,
-                           const int32_t *__restrict__ col, uint64_t seed,
-                           const int32_t *__restrict__ colour, int32_t *__restrict__ next) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    next[i] = -1;
-    if (colour[i] >= 0) continue;
-    const uint64_t pi = splitmix(seed, (uint64_t)i);
-    bool is_max = true;
-    uint64_t used = 0;
-    const int64_t b = rowptr[i], e = rowptr[i + 1];
-    for (int64_t k = b; k < e; ++k) {
-      const int64_t j = col[k];
-      if (j == i) continue;
-      const int32_t cj = colour[j];
-      if (cj < 0) {
-        const uint64_t pj = splitmix(seed, (uint64_t)j);
-        if (pj > pi || (pj == pi && j > i)) {
-          is_max = false;
-          break;
-        }
-      } else if (cj < 64) {
-        used |= 1ull << cj;
-      }
-    }
-    if (!is_max) continue;
-    int32_t c = 0;
-    for (;;) {
-      bool taken;
-      if (c < 64) {
-        taken = (used >> c) & 1ull;
-      } else {
-        taken = false;
-        for (int64_t k = b; k < e; ++k)
-          if (col[k] != i && colour[col[k]] == c) taken = true;
-      }
-      if (!taken) break;
-      ++c;
-    }
-    next[i] = c;
-  }
+// Jones-Plassmann colouring (see the oracle's lo_colour_jp): in a round a vertex
+// that beats all its uncoloured neighbours on (priority, index) takes the smallest
+// colour its coloured neighbours leave, as they stood before the round.
+//
+// Bound by the rounds (64 for 27 entries a row): a colour is kept with its round, so
+// that one launch a round can tell what the round wrote; a round's list holds the
+// vertices still without a colour, each with a neighbour that beat it, and most look
+// at that one alone.  G lanes share a row, 8 of them while many vertices are left and
+// 32 below kJpWide, where a round is as long as one row's chain of loads.  With all
+// rows in every round and the colours committed by a second launch, a setup and solve
+// of 998400 rows of 27 entries took 110.8 ms, now 108.8 (rounds of the finest level
+// 2.8 ms, of 6k to 170k rows 0.3 to 0.65).
+constexpr int kJpRounds = 8;  // rounds between two looks of the host at what remains
+constexpr int kJpWide = 32768;
+
+// the colour of a vertex before `round`, negative while it had none (low half:
+// colour, high half: its round; past L1, other vertices of the launch write)
+__device__ __forceinline__ int32_t jp_colour(const int64_t *p, int32_t round) {
+  int64_t v;
+  asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return (int32_t)(v >> 32) == round ? -1 : (int32_t)v;
 }
 
-// the round's colours, the vertices still without one and the highest colour
-// (one atomic per block: one per vertex on a single address serialised a round)
-__global__ void __launch_bounds__(256) k_jp_commit(int64_t n, int32_t *colour,
-                                                   const int32_t *next,
-                                                   unsigned long long *remaining, int *maxc) {
-  __shared__ int part[2][8];
-  int left = 0, top = -1;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t c = next[i];
-    if (c >= 0) {
-      colour[i] = c;
-      top = max(top, c);
-    } else {
-      left += colour[i] < 0;
+template <int G, bool FIRST>
+__global__ void __launch_bounds__(256) k_jp_round(
+  int64_t n, const int64_t *__restrict__ rowptr, const int32_t *__restrict__ col, uint64_t seed,
+  int64_t *state, int32_t round, unsigned long long *count, const int2 *__restrict__ list,
+  int2 *__restrict__ rest) {
+  __shared__ int2 kept[256 / G];
+  __shared__ int nkept;
+  __shared__ unsigned long long base;
+  if (threadIdx.x == 0) nkept = 0;
+  __syncthreads();
+  const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / G;
+  const int lane = threadIdx.x % G;
+  const unsigned group = G == 32 ? 0xffffffffu
+                                 : ((1u << (G % 32)) - 1) << (threadIdx.x / G * G % 32);
+  if (t < (FIRST ? n : (int64_t)count[0])) {
+    int2 v = FIRST ? make_int2((int)t, -1) : list[t];
+    const int64_t i = v.x;
+    if (FIRST || jp_colour(state + v.y, round) >= 0) {
+      v.y = -1;
+      const int64_t b = rowptr[i], e = rowptr[i + 1];
+      const uint64_t pi = splitmix(seed, (uint64_t)i);
+      uint64_t used = 0;  // colours below 64
+      for (int64_t k0 = b; k0 < e && v.y < 0; k0 += G) {
+        const int64_t k = k0 + lane, j = k < e ? (int64_t)col[k] : i;
+        bool beaten = false;
+        if (j != i) {
+          const int32_t cj = FIRST ? -1 : jp_colour(state + j, round);
+          const uint64_t pj = splitmix(seed, (uint64_t)j);
+          if (cj < 0) beaten = pj > pi || (pj == pi && j > i);
+          else if (cj < 64) used |= 1ull << cj;
+        }
+        const unsigned m = __ballot_sync(group, beaten) & group;
+        if (m) v.y = (int)__shfl_sync(group, (int)j, __ffs(m) - 1);
+      }
+      if (v.y < 0) {
+        int32_t c = 0;
+        for (int32_t c0 = 0;; c0 += 64) {
+          if (c0) {
+            used = 0;
+            for (int64_t k = b + lane; k < e; k += G) {
+              if (col[k] == i) continue;
+              const int32_t cj = jp_colour(state + col[k], round) - c0;
+              if (cj >= 0 && cj < 64) used |= 1ull << cj;
+            }
+          }
+          const uint64_t lo = __reduce_or_sync(group, (unsigned)used);
+          const uint64_t all = (uint64_t)__reduce_or_sync(group, (unsigned)(used >> 32)) << 32 | lo;
+          c = c0 + __ffsll((long long)~all) - 1;
+          if (~all) break;
+        }
+        if (lane == 0) {
+          const int64_t w = (int64_t)round << 32 | c;
+          asm volatile("st.relaxed.gpu.global.s64 [%0], %1;" ::"l"(state + i), "l"(w) : "memory");
+        }
+      }
     }
-  }
-  left = __reduce_add_sync(0xffffffffu, left);
-  top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0) {
-    part[0][threadIdx.x >> 5] = left;
-    part[1][threadIdx.x >> 5] = top;
+    if (v.y >= 0 && lane == 0) kept[atomicAdd(&nkept, 1)] = v;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) {
-      left += part[0][w];
-      top = max(top, part[1][w]);
-    }
-    if (left) atomicAdd(remaining, (unsigned long long)left);
-    if (top >= 0) atomicMax(maxc, top);
-  }
+  if (nkept == 0) return;
+  if (threadIdx.x == 0) base = atomicAdd(count + 1, (unsigned long long)nkept);
+  __syncthreads();
+  if ((int)threadIdx.x < nkept) rest[base + threadIdx.x] = kept[threadIdx.x];
 }
 
-// rounds launched between two looks at what remains: a round with nothing left
-// changes nothing, and a look costs the host about 20 us.  170k rows: 3.8 -> 2.4 ms
-// with the order below
-constexpr int kJpRounds = 4;
+__global__ void __launch_bounds__(256) k_jp_colours(int64_t n, const int64_t *__restrict__ state,
+                                                    int32_t *__restrict__ colour, int *maxc) {
+  int top = -1;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    colour[i] = (int32_t)state[i];
+    top = max(top, colour[i]);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top >= 0) atomicMax(maxc, top);
+}
 
 lgx_status colouring_jp(const Csr &a, uint64_t seed, cudaStream_t s, DBuf<int32_t> &colour,
                         int32_t &ncolours) {
   const int64_t n = a.n;
   LGX_CHECK(colour.alloc(n));
-  DBuf<int32_t> next;
-  DBuf<unsigned long long> rem;
-  DBuf<int> maxc;
-  LGX_CHECK(next.alloc(n));
-  LGX_CHECK(rem.alloc(1));
-  LGX_CHECK(maxc.alloc(1));
-  LGX_CUDA(cudaMemsetAsync(colour.p, 0xFF, sizeof(int32_t) * std::max<int64_t>(n, 1), s));
-  LGX_CUDA(cudaMemsetAsync(maxc.p, 0xFF, sizeof(int), s));
-  const unsigned g = (unsigned)std::min<int64_t>(grid_for(n, 256), 16384);
+  // states, two lists, the rounds' list lengths and the highest colour
+  DBuf<int64_t> work;
+  LGX_CHECK(work.alloc(3 * n + kJpRounds + 2));
+  int64_t *state = work.p;
+  int2 *list[2] = {reinterpret_cast<int2 *>(work.p + n), reinterpret_cast<int2 *>(work.p + 2 * n)};
+  unsigned long long *count = reinterpret_cast<unsigned long long *>(work.p + 3 * n);
+  int *maxc = reinterpret_cast<int *>(count + kJpRounds + 1);
+  LGX_CUDA(cudaMemsetAsync(state, 0xFF, sizeof(int64_t) * n, s));
+  LGX_CUDA(cudaMemsetAsync(maxc, 0xFF, sizeof(int), s));
   unsigned long long h_rem = (unsigned long long)n;
-  int64_t rounds = 0;
+  int32_t round = 0;
   while (h_rem > 0) {
-    if ((rounds += kJpRounds) > n + kJpRounds)
-      return fail(LGX_ERR_INVALID, "colouring did not terminate");
-    for (int q = 0; q < kJpRounds; ++q) {
-      k_jp_round<<<g, 256, 0, s>>>(n, a.rowptr.p, a.col.p, seed, colour.p, next.p);
-      LGX_LAUNCH_CHECK();
-      if (q == kJpRounds - 1)
-        LGX_CUDA(cudaMemsetAsync(rem.p, 0, sizeof(unsigned long long), s));
-      k_jp_commit<<<g, 256, 0, s>>>(n, colour.p, next.p, rem.p, maxc.p);
+    // a round colours at least the first of the remaining vertices
+    if (round > n) return fail(LGX_ERR_INVALID, "colouring did not terminate");
+    LGX_CUDA(cudaMemcpyAsync(count, &h_rem, sizeof(h_rem), cudaMemcpyHostToDevice, s));
+    LGX_CUDA(cudaMemsetAsync(count + 1, 0, sizeof(unsigned long long) * kJpRounds, s));
+    const bool wide = h_rem < kJpWide;
+    const unsigned g = (unsigned)((h_rem * (wide ? 32 : 8) + 255) / 256);
+    for (int q = 0; q < kJpRounds; ++q, ++round) {
+      auto *kern = round == 0 ? (wide ? k_jp_round<32, true> : k_jp_round<8, true>)
+                              : (wide ? k_jp_round<32, false> : k_jp_round<8, false>);
+      kern<<<g, 256, 0, s>>>(n, a.rowptr.p, a.col.p, seed, state, round, count + q,
+                             list[round & 1], list[(round + 1) & 1]);
       LGX_LAUNCH_CHECK();
     }
-    LGX_CUDA(cudaMemcpyAsync(&h_rem, rem.p, sizeof(h_rem), cudaMemcpyDeviceToHost, s));
+    LGX_CUDA(cudaMemcpyAsync(&h_rem, count + kJpRounds, sizeof(h_rem), cudaMemcpyDeviceToHost, s));
     LGX_CUDA(cudaStreamSynchronize(s));
   }
+  if (n > 0) {
+    k_jp_colours<<<(unsigned)std::min<int64_t>(grid_for(n, 256), 16384), 256, 0, s>>>(
+        n, state, colour.p, maxc);
+    LGX_LAUNCH_CHECK();
+  }
   int h_max = -1;
-  LGX_CUDA(cudaMemcpyAsync(&h_max, maxc.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  LGX_CUDA(cudaMemcpyAsync(&h_max, maxc, sizeof(int), cudaMemcpyDeviceToHost, s));
   LGX_CUDA(cudaStreamSynchronize(s));
   ncolours = h_max + 1;
   return LGX_OK;

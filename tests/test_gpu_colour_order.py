@@ -48,3 +48,41 @@ def test_colour_order(cuda, n, ncolours):
     colours[n // 2] = ncolours
     with pytest.raises(cuda.LinealError):
         cuda.Colouring.from_array(m, colours, ncolours)
+
+
+def _pattern(kind):
+    """A clique of 70 rows within 300 (more than 64 colours, rows of 1 and of 70
+    entries), or random rows with a few one-sided
+    couplings."""
+    rng = np.random.default_rng(21)
+    if kind == "clique":
+        n, member = 300, np.zeros(300, dtype=bool)
+        member[rng.permutation(300)[:70]] = True
+        dense = np.outer(member, member) | np.eye(300, dtype=bool)
+    else:
+        n = 1500
+        upper = np.triu(rng.random((n, n)) < 0.005, 1)
+        dense = upper | upper.T | np.eye(n, dtype=bool)
+        one_sided = rng.integers(0, n, (2, 3))
+        dense[one_sided[0], one_sided[1]] = True
+    r, c = np.nonzero(dense)
+    rowptr = np.zeros(n + 1, dtype=np.int64)
+    np.cumsum(np.bincount(r, minlength=n), out=rowptr[1:])
+    return lo.Csr(rowptr, c.astype(np.int32), np.ones(len(r)), symmetric=False), dense
+
+
+@pytest.mark.parametrize("kind,seed", [("clique", 1), ("clique", 2), ("unsymmetric", 1),
+                                       ("unsymmetric", 2), ("unsymmetric", 4)])
+def test_jp_patterns(cuda, kind, seed):
+    ref, dense = _pattern(kind)
+    m = cuda.CsrMatrix.from_host(ref.rowptr, ref.col, ref.val, symmetric=False)
+    want, nc = lo.colour_jp(ref, seed)
+    same = want[:, None] == want[None, :]
+    np.fill_diagonal(same, False)
+    if (same & dense).any():  # a one-sided neighbour took the colour in the same round
+        with pytest.raises(cuda.LinealError):
+            cuda.Colouring.jp(m, seed=seed)
+        return
+    got, gnc = cuda.Colouring.jp(m, seed=seed).export()
+    assert gnc == nc
+    np.testing.assert_array_equal(got.cpu().numpy(), want)
