@@ -327,11 +327,14 @@ __host__ __device__ constexpr size_t wstage_bytes(int capw, size_t vsize) {
   return (size_t)(kWarpTileRows + 4) * 8 + (size_t)(capw + 8) * 4 + (size_t)(capw + 8) * vsize;
 }
 // per CTA: WPC * S barriers and WPC * S "unstaged" flags, then the stages
+// (XB bytes of gathered vector per entry follow the stages, see kSpreadMb)
 __host__ __device__ constexpr size_t wheader_bytes(int wpc, int nst) {
   return (((size_t)wpc * nst * 12) + 15) & ~(size_t)15;
 }
-__host__ __device__ constexpr size_t wsmem_bytes(int wpc, int nst, int capw, size_t vsize) {
-  return wheader_bytes(wpc, nst) + (size_t)wpc * nst * wstage_bytes(capw, vsize);
+__host__ __device__ constexpr size_t wsmem_bytes(int wpc, int nst, int capw, size_t vsize,
+                                                 size_t xsize = 0) {
+  return wheader_bytes(wpc, nst) +
+         (size_t)wpc * nst * (wstage_bytes(capw, vsize) + (size_t)(capw + 8) * xsize);
 }
 
 // one-warp CTAs per SM that the registers of rows in rounds of 32, 16 and 8
@@ -339,6 +342,20 @@ __host__ __device__ constexpr size_t wsmem_bytes(int wpc, int nst, int capw, siz
 constexpr int kSmallMb32 = 10, kSmallMb16 = 14, kSmallMb8 = 20;
 // four-warp CTAs per SM of products whose rows have at most 8 entries
 constexpr int kShortMb = 6;
+// one-warp CTAs whose lanes gather a tile's entries in storage order into
+// shared memory, before each lane runs its row (launch_spread)
+constexpr int kSpreadMb = 16;
+
+// one vector entry into shared memory
+template <typename T>
+__device__ __forceinline__ void copy_async(T *dst, const T *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src),
+               "n"((int)sizeof(T))
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
 
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -383,6 +400,12 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
     r.val = reinterpret_cast<VT *>(p + (size_t)(kWarpTileRows + 4) * 8 + (size_t)(capw + 8) * 4);
     return r;
   };
+  constexpr bool SPREAD = MB == kSpreadMb;
+  typename Op::X *xs = nullptr;
+  if constexpr (SPREAD) {
+    static_assert(WPC == 1 && S == 1, "one warp, one stage");
+    xs = reinterpret_cast<typename Op::X *>(smem_raw + wheader_bytes(1, 1) + sb);
+  }
   const int64_t ntiles = (re - rb + kWarpTileRows - 1) / kWarpTileRows;
   const int64_t GW = (int64_t)gridDim.x * WPC;
   int64_t t = (int64_t)blockIdx.x * WPC + warp;
@@ -449,7 +472,20 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
       const int64_t p0 = r0 & ~1ll;
       const int64_t e0 = sg.rp[r0 - p0];
       const int64_t c0 = e0 & ~(CA - 1), v0 = e0 & ~(VA - 1);
-      if (row < r1) {
+      if constexpr (SPREAD) {
+        const int n = (int)(sg.rp[r1 - p0] - e0);
+        const int32_t *c = sg.col + (e0 - c0);
+#pragma unroll 8
+        for (int k = lane; k < n; k += 32) copy_async(xs + k, op.x + c[k]);
+        typename Op::Pre pre{};
+        if (row < r1) pre = op.begin(row, i);
+        copy_async_wait();
+        __syncwarp();
+        if (row < r1) {
+          const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
+          op.staged(pre, i, sg.col + (b - c0), sg.val + (b - v0), xs + (b - e0), (int)(e - b));
+        }
+      } else if (row < r1) {
         const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
         contrib += run_row<W, FLAT>(op, row, i, sg.col + (b - c0), sg.val + (b - v0),
                                     (int)(e - b));
@@ -512,7 +548,8 @@ inline lgx_status launch_wrows(int64_t rb, int64_t re, const Csr &a, const VT *v
   const int64_t mw = a.max_win > 4 ? a.max_win : 4;
   if (mw > (1 << 20)) return LGX_OK;
   const int capw = (int)((mw + 7) & ~7ll);  // 16-byte value spans also for 2-byte values
-  const size_t smem = wsmem_bytes(WPC, S, capw, sizeof(VT));
+  const size_t smem =
+    wsmem_bytes(WPC, S, capw, sizeof(VT), MB == kSpreadMb ? sizeof(typename Op::X) : 0);
   if (smem > (size_t)kWrowsSmemMax) return LGX_OK;  // too long rows: CTA tiles
   static const cudaError_t attr = cudaFuncSetAttribute(
     k_wrows<VT, Op, WPC, S, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWrowsSmemMax);
@@ -597,6 +634,39 @@ inline lgx_status launch_small(int64_t rb, int64_t re, const Csr &a, const VT *v
   return launch_wrows<VT, Op, 1, 1, kSmallMb32>(rb, re, a, val, op, s, done);
 }
 
+// operations with a staged form (Op::Pre, begin, staged, spread)
+template <class Op, class = void>
+struct StagedForm {
+  static constexpr bool value = false;
+};
+template <class Op>
+struct StagedForm<Op, std::void_t<typename Op::Pre>> {
+  static constexpr bool value = true;
+};
+
+// Listed rows (colours of levels in natural order) in few tiles, with the lanes
+// along the entries.  With a lane per row, the k-th entries of 32 rows of one
+// colour lie in about 24 lines of x, and with the bank conflicts of the rows'
+// columns and values (35 wavefronts an entry) the L1 bounds the launch, as do
+// its two or three rounds of gathers; lanes along the entries of a row meet
+// about 15 lines, all gathers of a tile are in flight at once, and short rows
+// leave no lane idle.  The arithmetic is the row's own.  Against that stand 8
+// (float 4) more bytes of shared memory an entry, so fewer warps: beyond eight
+// tiles per SM the plain form wins.  AMG-CG at 256^3, 27 points, FP64: 438 ->
+// 428 ms (all launches spread 433, from eight tiles on only 442); float
+// vectors, 121 x 117 x 125, 27 points: 65.1 -> 63.9; float rows of up to 16
+// entries on average lose (256^3, 7 points: 289 -> 292).
+template <typename VT, class Op>
+inline lgx_status launch_spread(int64_t rb, int64_t re, const Csr &a, const VT *val, const Op &op,
+                                cudaStream_t s, bool *done) {
+  if constexpr (StagedForm<Op>::value && !kIsBf16<VT>) {
+    if (op.spread() && re - rb <= (int64_t)sm_count() * 8 * kWarpTileRows &&
+        (sizeof(typename Op::X) == 8 || a.nnz > 16 * a.n))
+      return launch_wrows<VT, Op, 1, 1, kSpreadMb>(rb, re, a, val, op, s, done);
+  }
+  return LGX_OK;
+}
+
 // rows [rb, re) of `a` (values `val`) through the engine configuration the
 // autotuner chose for this matrix and operation, else the process-wide one
 template <typename VT, class Op>
@@ -607,7 +677,10 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
   const int tuned = a.tuned[TuneClass<Op>::value][tune_value_index<VT>()];
   const int cfg = tuned >= 0 ? tuned : rows_config();
   if constexpr (!Op::kReduce) {  // (a reduction wants few, large CTAs)
-    if (cfg == 3 || cfg == 7) LGX_CHECK((launch_small<VT, Op>(rb, re, a, val, op, s, &done)));
+    if (cfg == 3 || cfg == 7) {
+      LGX_CHECK((launch_spread<VT, Op>(rb, re, a, val, op, s, &done)));
+      if (!done) LGX_CHECK((launch_small<VT, Op>(rb, re, a, val, op, s, &done)));
+    }
     if (done) return LGX_OK;
   }
   // rows of at most 8 entries (7-point operators) at 256^3: FP64 product 350

@@ -733,6 +733,27 @@ struct SorOp {
     x[i] = sor_value<XT>(accum, diag, xi, y, relax, m1, ultra, relax_one);
     return 0.0;
   }
+  // the row from gathered entries (natural-order rows, xs[k] = x[c[k]])
+  bool spread() const { return rows && !from_zero; }
+  struct Pre {
+    XT b, xi;
+    double y;
+  };
+  __device__ __forceinline__ Pre begin(int64_t r, int32_t i) const {
+    return {b[i], x[i], sizeof(XT) == 8 && rdiag ? rdiag[r] : 0.0};
+  }
+  __device__ __forceinline__ void staged(const Pre &p, int32_t i, const int32_t *c, const VT *v,
+                                         const XT *xs, int len) const {
+    XT accum = p.b, diag = XT(0);
+#pragma unroll 4
+    for (int k = 0; k < len; ++k) {
+      const XT a = cvt<XT>(v[k]);
+      const bool own = c[k] == i;
+      if (own) diag = a;
+      if (!own || ultra) accum = fma(-a, xs[k], accum);
+    }
+    x[i] = sor_value<XT>(accum, diag, p.xi, p.y, relax, m1, ultra, relax_one);
+  }
   // bfloat16 values v with a_ij = s_i v_ij: accum = b_i - s_i sum_{j != i} v_ij x_j,
   // a_ii = s_i v_ii (float arithmetic; a precision-form smoother, not the
   // reference's bits)
@@ -812,6 +833,21 @@ struct SorLoOp {
     x[i] = sor_value<XT>(accum, diag, XT(0), y, relax, m1, ultra, relax_one);
     return 0.0;
   }
+  bool spread() const { return rows != nullptr; }
+  struct Pre {
+    XT b, diag;
+    double y;
+  };
+  __device__ __forceinline__ Pre begin(int64_t r, int32_t i) const {
+    return {b[i], (XT)pdiag[r], sizeof(XT) == 8 && rdiag ? rdiag[r] : 0.0};
+  }
+  __device__ __forceinline__ void staged(const Pre &p, int32_t i, const int32_t *, const VT *v,
+                                         const XT *xs, int len) const {
+    XT accum = p.b;
+#pragma unroll 4
+    for (int k = 0; k < len; ++k) accum = fma(-cvt<XT>(v[k]), xs[k], accum);
+    x[i] = sor_value<XT>(accum, p.diag, XT(0), p.y, relax, m1, ultra, relax_one);
+  }
   __device__ __forceinline__ void finish(double) const {}
 };
 
@@ -832,6 +868,18 @@ struct ListResidualOp {
     const XT ax = row_dot<W, FLAT, VT, XT>(c, v, len, x, XT(0));
     r[i] = UP ? -ax : b[i] - ax;
     return 0.0;
+  }
+  bool spread() const { return rows != nullptr; }
+  struct Pre {
+    XT b;
+  };
+  __device__ __forceinline__ Pre begin(int64_t, int32_t i) const { return {UP ? XT(0) : b[i]}; }
+  __device__ __forceinline__ void staged(const Pre &p, int32_t i, const int32_t *, const VT *v,
+                                         const XT *xs, int len) const {
+    XT ax = XT(0);
+#pragma unroll 4
+    for (int k = 0; k < len; ++k) ax = fma(cvt<XT>(v[k]), xs[k], ax);
+    r[i] = UP ? -ax : p.b - ax;
   }
   __device__ __forceinline__ void finish(double) const {}
 };
