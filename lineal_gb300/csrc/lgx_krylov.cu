@@ -694,7 +694,7 @@ static lgx_status krylov_create(int kind, const lgx_matrix *a, const double *d_b
 // behind it instead of after a gap of 10 to 25 us.  What the direction itself can
 // end the solve with (rho, flags) the next update sees on the device (gate).
 // SSOR-CG, 7 points: 14 x 17 x 18 4.62 -> 3.97 ms, 84^3 44.4 -> 39.8; 27 points,
-// 30 x 31 x 33: 14.8 -> 13.7, 66 x 65 x 67: 47.6 -> 45.9.  The refinement's float
+// 30 x 31 x 33: 14.8 -> 13.7, 61 x 67 x 71: 47.6 -> 45.9.  The refinement's float
 // iterations gained nothing from it (66.0 / 66.1 ms) and look at their ends.
 static lgx_status run_overlapped(lgx_krylov &K, double &res, double *history) {
   const lgx_solve_params &p = K.p;
