@@ -689,6 +689,17 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
     LGX_CHECK((launch_wrows<VT, Op, 4, 1, kShortMb>(rb, re, a, val, op, s, &done)));
     if (done) return LGX_OK;
   }
+  // Larger colours of natural-order levels with long rows (over 16 entries on
+  // average, 8 of a half): eight-warp CTAs, 16 gathers a round, two per SM --
+  // with 16 instead of 20 staged warps more of the SM caches x, of which 32 such
+  // rows read hundreds of lines, and a row has fewer rounds.  AMG-CG at 256^3,
+  // 27 points, FP64: 429 -> 419 ms; float vectors, 121 x 117 x 125, 27 points:
+  // 64.3 -> 57.0; shorter rows (256^3, 7 points) the same or slower (290 / 292).
+  if constexpr (StagedForm<Op>::value && TuneClass<Op>::value == 1) {
+    if (tuned < 0 && cfg == 3 && op.spread() && a.nnz > Op::kLongRow * a.n)
+      LGX_CHECK((launch_wrows<VT, Op, 8, 1>(rb, re, a, val, op, s, &done)));
+    if (done) return LGX_OK;
+  }
   switch (cfg) {
     case 3: LGX_CHECK((launch_wrows<VT, Op, 4, 1>(rb, re, a, val, op, s, &done))); break;
     case 4: LGX_CHECK((launch_wrows<VT, Op, 4, 2>(rb, re, a, val, op, s, &done))); break;

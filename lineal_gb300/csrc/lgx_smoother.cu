@@ -734,6 +734,7 @@ struct SorOp {
     return 0.0;
   }
   // the row from gathered entries (natural-order rows, xs[k] = x[c[k]])
+  static constexpr int kLongRow = 16;  // entries on average (launch_rows)
   bool spread() const { return rows && !from_zero; }
   struct Pre {
     XT b, xi;
@@ -833,6 +834,7 @@ struct SorLoOp {
     x[i] = sor_value<XT>(accum, diag, XT(0), y, relax, m1, ultra, relax_one);
     return 0.0;
   }
+  static constexpr int kLongRow = 8;  // half rows
   bool spread() const { return rows != nullptr; }
   struct Pre {
     XT b, diag;

@@ -1,7 +1,10 @@
 """Rows of natural-order levels with the lanes along their entries: V-cycles bit
 for bit against the engine configuration that gives every row a lane, and the
 FP64 ones against the oracle; rows of 1 to 41 entries, one row longer than the
-rest of its tile, sizes around a tile of 32 rows and around eight tiles per SM."""
+rest of its tile, sizes around a tile of 32 rows and around eight tiles per SM
+(beyond them long rows run in eight-warp CTAs)."""
+
+import functools
 
 import numpy as np
 import pytest
@@ -13,6 +16,7 @@ pytestmark = pytest.mark.gpu
 PARAMS = dict(min_coarsen_size=16, partition_size=512)
 
 
+@functools.lru_cache(maxsize=1)
 def _matrix(n, longest, seed, wide=0):
     """Symmetric M-matrix of bands at a spread of offsets, some rows cut to
     their diagonal; row n / 2 coupled to `wide` others."""
@@ -41,9 +45,10 @@ def _matrix(n, longest, seed, wide=0):
     return lo.Csr(rowptr, c.astype(np.int32), v, symmetric=True)
 
 
-@pytest.mark.parametrize("n,longest,wide", [(31, 5, 0), (33, 9, 0), (640, 41, 0), (3000, 33, 900),
-                                            (20000, 19, 0), (90000, 7, 0), (90000, 21, 0)])
 @pytest.mark.parametrize("form", ["fp64", "f32", "coarse_f32"])
+@pytest.mark.parametrize("n,longest,wide", [(31, 5, 0), (33, 9, 0), (640, 41, 0), (3000, 33, 900),
+                                            (20000, 19, 0), (90000, 7, 0), (90000, 21, 0),
+                                            (500000, 23, 0)])
 def test_spread_rows_vcycle(cuda, n, longest, wide, form):
     ref = _matrix(n, longest, 31, wide)
     m = cuda.CsrMatrix.from_host(ref.rowptr, ref.col, ref.val, symmetric=True)
