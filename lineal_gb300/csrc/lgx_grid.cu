@@ -718,9 +718,13 @@ __global__ void __launch_bounds__(256, PTS == 27 ? 4 : 6)
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned c0 = (unsigned)t0 / (unsigned)g.block, c1 = (unsigned)t1 / (unsigned)g.block;
-    const unsigned need = g_parts<PTS, UP>((int)c0) | g_parts<PTS, UP>((int)c1);
     if constexpr (PTS == 27) {
+      // the groups of every colour in the tile: on small grids it spans more than
+      // two, and one in the middle can need a group that the outer ones do not
+      const unsigned c1 = (unsigned)t1 / (unsigned)g.block;
+      unsigned need = 0u;
+      for (unsigned c = (unsigned)t0 / (unsigned)g.block; c <= c1; ++c)
+        need |= g_parts<PTS, UP>((int)c);
       const unsigned planes = (need & 4u ? 18u : 0u) + (need & 2u ? 6u : 0u) +
                               (need & 1u ? 3u : UP ? 0u : 1u);
       mbar_expect_tx(&bar, planes * RT * (unsigned)sizeof(float));
