@@ -80,6 +80,14 @@ struct SoloShared {
 
 __device__ __forceinline__ bool finite_bits(double v) { return exponent_field(v) != 0x7ff; }
 
+// What ||r||^2 has to exceed for ||r|| > limit (a square root is a chain of its own
+// in every iteration): the limit's square rounded down, so that neither a tiny nor
+// a huge one changes the answer; nothing is at or below a negative limit, and
+// nothing beyond one that is not a number.
+__device__ __forceinline__ double stop_square(double limit) {
+  return limit < 0.0 ? -1.0 : __dmul_rd(limit, limit);
+}
+
 // The barrier of the whole grid and the reductions that end in it.  A reduction
 // leaves its CTA's sums in the barrier's parity of A.part, arrives on one counter
 // and, when all have arrived, adds the sums of all CTAs.  (Polling every CTA's
@@ -231,7 +239,6 @@ __global__ void __launch_bounds__(kST, 2) k_solo_cg(SoloArgs A) {
   const int first = lo + (int)threadIdx.x;
   double one[1], two[2] = {0.0, 0.0};
   auto go_on = [&]() {
-    // ||r|| > rtol ||r0|| in squares (a square root is a chain of its own)
     sh.go = sh.flag == 0 && sh.it < A.maxit && sh.res2 > sh.stop2 && sh.rho != 0.0;
   };
   // r = b - A x, p = z = M r, rho = r.z
@@ -252,7 +259,7 @@ __global__ void __launch_bounds__(kST, 2) k_solo_cg(SoloArgs A) {
         sh.res2 = s[0];
         sh.rho = precon ? s[1] : s[0];
         sh.r0 = sqrt(s[0]);
-        sh.stop2 = (A.rtol * sh.r0) * (A.rtol * sh.r0);
+        sh.stop2 = stop_square(A.rtol * sh.r0);
         sh.it = 0;
         sh.flag = finite_bits(s[0]) && finite_bits(sh.rho) ? 0 : 4;
         go_on();
@@ -337,7 +344,6 @@ __global__ void __launch_bounds__(kST, 2) k_solo_bicgstab(SoloArgs A) {
   const int first = lo + (int)threadIdx.x;
   double one[1] = {0.0}, two[2];
   auto go_on = [&]() {
-    // ||r|| > rtol ||r0|| in squares (a square root is a chain of its own)
     sh.go = sh.flag == 0 && sh.it < A.maxit && sh.res2 > sh.stop2 && sh.rho != 0.0;
   };
   // r = b - A x, r0 = p = r, rho = ||r||^2
@@ -356,7 +362,7 @@ __global__ void __launch_bounds__(kST, 2) k_solo_bicgstab(SoloArgs A) {
   if (!grid.reduce(one, [&](const double (&s)[1]) {
         sh.res2 = sh.rho = s[0];
         sh.r0 = sqrt(s[0]);
-        sh.stop2 = (A.rtol * sh.r0) * (A.rtol * sh.r0);
+        sh.stop2 = stop_square(A.rtol * sh.r0);
         sh.it = 0;
         sh.flag = finite_bits(s[0]) ? 0 : 4;
         go_on();
