@@ -470,13 +470,25 @@ bool overlap(const void *a, const void *b, size_t bytes) {
 }  // namespace
 
 // Runs the solve when the system is one for this path (*done), else leaves it.
-// Where the line lies: beyond, an iteration is bound by bandwidth, and the
-// launches' own kernels stream better than this one's plain loops.  50 Jacobi-CG
-// iterations, setup included, launches / one launch, ms: lookup stencil 24^3 2.2 /
-// 0.8, 64^3 3.3 / 1.4, 96^3 4.9 / 2.8, 112^3 6.6 / 4.2, 128^3 8.2 / 8.5; 7-point
-// CSR 64^3 3.3 / 1.5, 112^3 7.2 / 5.0, 128^3 9.2 / 9.1; 27-point CSR 64^3 4.1 /
-// 2.7, 96^3 7.9 / 7.2, 112^3 (37M entries) 10.7 / 11.0.
-constexpr int64_t kSoloMaxRows = 1500000, kSoloMaxEntries = 25000000;
+// Where the line lies: beyond kSoloMaxRows rows or kSoloMaxEntries entries an
+// iteration is bound by bandwidth, and the launches' own kernels stream better than
+// this one's plain loops.  50 Jacobi-CG iterations, setup included, launches / one
+// launch, ms: lookup stencil 24^3 2.2 / 0.8, 64^3 3.3 / 1.4, 96^3 4.9 / 2.8, 112^3
+// 6.6 / 4.2, 128^3 8.2 / 8.5; 7-point CSR 64^3 3.3 / 1.5, 112^3 7.2 / 5.0, 128^3 9.2
+// / 9.1; 27-point CSR 64^3 4.1 / 2.7, 96^3 7.9 / 7.2, 104^3 (30M entries) 9.3 / 8.8,
+// 108^3 (33M) 10.0 / 9.8, 112^3 (37M) 10.7 / 10.7 (BiCGStab 16.5 / 16.2, 17.8 /
+// 18.0, 19.4 / 19.7).
+constexpr int64_t kSoloMaxRows = 1500000, kSoloMaxEntries = 32000000;
+// A thread works its rows entry by entry, about 0.18 us each, and all CTAs wait for
+// the slowest: a chain of up to kSoloChain entries per product, and one more for
+// every kSoloChainStep entries of the matrix (which the launches have to stream),
+// beats the launches.  The chain is bounded by the longest row, so a few long rows
+// leave the system to the launches, and no barrier waits for more than 0.4 ms of
+// work.  50 Jacobi-CG iterations, launches / one launch, ms, even rows: 2000 rows
+// of 30 entries 2.7 / 1.3, of 100 2.8 / 2.7, of 400 3.7 / 8.0; 5000 of 200 3.0 /
+// 4.5; 20000 of 60 2.8 / 1.9, of 200 3.8 / 4.5; 100000 of 100 6.2 / 3.9, of 200
+// 10.7 / 6.8; 300000 of 80 10.4 / 6.8.
+constexpr int64_t kSoloChain = 192, kSoloChainStep = 20000;
 
 lgx_status solo_solve(bool cg, const lgx_matrix *a, const double *d_b, double *d_x,
                       const lgx_solve_params *p, cudaStream_t s, int64_t *iterations,
@@ -509,11 +521,15 @@ lgx_status solo_solve(bool cg, const lgx_matrix *a, const double *d_b, double *d
     else LGX_CHECK(solo_kernel<S_VALUE>(cg, n, &fn, &most));
   }
   if (most < 1) return LGX_OK;
-  if (p->precon == LGX_PRECON_JACOBI)
-    LGX_CHECK(matrix_diagonal(const_cast<lgx_matrix *>(a), s, &A.diag));
   const int64_t ctas = std::min<int64_t>(most, std::max<int64_t>(1, n / kSoloMinRows));
   A.n = (int)n;
   A.chunk = (int)(((n + ctas - 1) / ctas + 31) / 32 * 32);
+  if (a->kind == LGX_MATRIX_CSR &&
+      (a->csr.nnz > kSoloMaxEntries ||
+       (A.chunk + kST - 1) / kST * a->csr.max_row > kSoloChain + a->csr.nnz / kSoloChainStep))
+    return LGX_OK;
+  if (p->precon == LGX_PRECON_JACOBI)
+    LGX_CHECK(matrix_diagonal(const_cast<lgx_matrix *>(a), s, &A.diag));
   const unsigned grid = (unsigned)((n + A.chunk - 1) / A.chunk);
   DBuf<double> ws, hist;
   DBuf<double> part;
