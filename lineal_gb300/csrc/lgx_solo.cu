@@ -76,7 +76,15 @@ struct SoloShared {
   double alpha, beta, omega, rho, res2, r0, stop2;
   int64_t it;
   int flag, go, rere, lost;
+  int huge;  // some CTA met an entry of 2^501 or more
 };
+
+// Up to kSoloMaxRows entries below 2^501 have a finite sum of squares.  BiCGStab
+// takes the norm of its half residual only where there are larger ones (for its
+// error on overflow); that there are travels as the top bit of the barriers'
+// counter, which counts to less than 2^31 (at most a million iterations).
+constexpr int kSoloHuge = 1023 + 501;
+constexpr unsigned kSoloHugeBit = 0x80000000u;
 
 __device__ __forceinline__ bool finite_bits(double v) { return exponent_field(v) != 0x7ff; }
 
@@ -94,26 +102,31 @@ __device__ __forceinline__ double stop_square(double limit) {
 // sums directly, marked with the barrier's number, saves the counter's round trip
 // and loses more to 152 warps reading 600 words that are being written: Jacobi-CG
 // at 64^3 36 us per iteration instead of 21.)
+// HUGE: the counter may carry kSoloHugeBit.  It is raised and looked at in one kind
+// of barrier only, sync_huge; a CTA that is still in the barrier before it when
+// another one raises the bit ignores it there and finds it here.
+template <bool HUGE>
 struct SoloGrid {
   const SoloArgs &A;
   SoloShared &sh;
   unsigned epoch;
   __device__ SoloGrid(const SoloArgs &a, SoloShared &s) : A(a), sh(s), epoch(0) {}
   // one thread, after a CTA barrier: arrive, wait for all
-  __device__ __forceinline__ void arrive_and_wait() {
+  __device__ __forceinline__ unsigned arrive_and_wait() {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(A.arrived) : "memory");
     const unsigned target = epoch * gridDim.x;
     const long long start = clock64();
     unsigned seen;
     for (;;) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(A.arrived) : "memory");
-      if (seen >= target) break;
+      if ((HUGE ? seen & ~kSoloHugeBit : seen) >= target) break;
       if (clock64() - start > (1ll << 31)) {
         sh.lost = 1;
         atomicExch(A.err, 1);
         break;
       }
     }
+    return seen;
   }
   // warp 0, after a CTA barrier: every CTA's r (of lane 0) summed (lane-strided,
   // then a tree) in all lanes
@@ -151,6 +164,19 @@ struct SoloGrid {
     if (gridDim.x > 1) {
       ++epoch;
       if (threadIdx.x == 0) arrive_and_wait();
+      __syncthreads();
+    }
+    return !sh.lost;
+  }
+  // sync, after which sh.huge says whether any thread of the grid has set it
+  __device__ __forceinline__ bool sync_huge() {
+    __syncthreads();
+    if (gridDim.x > 1) {
+      ++epoch;
+      if (threadIdx.x == 0) {
+        if (sh.huge) atomicOr(A.arrived, kSoloHugeBit);
+        if (arrive_and_wait() & kSoloHugeBit) sh.huge = 1;
+      }
       __syncthreads();
     }
     return !sh.lost;
@@ -228,7 +254,7 @@ __device__ __forceinline__ double solo_jacobi(const SoloArgs &A, double r, doubl
 template <int OP>
 __global__ void __launch_bounds__(kST, 2) k_solo_cg(SoloArgs A) {
   __shared__ SoloShared sh;
-  SoloGrid grid(A, sh);
+  SoloGrid<false> grid(A, sh);
   if (threadIdx.x == 0) sh.lost = 0;
   if (threadIdx.x < 48) sh.conn[threadIdx.x] = A.st.conn[threadIdx.x];
   __syncthreads();
@@ -308,7 +334,10 @@ __global__ void __launch_bounds__(kST, 2) k_solo_cg(SoloArgs A) {
     if (!grid.reduce(two, [&](const double (&s)[2]) {
           const double rho = precon ? s[1] : s[0];
           sh.res2 = s[0];
-          if (!finite_bits(s[0]) || !finite_bits(rho)) sh.flag |= 2;
+          // (a recomputed residual's norm is looked at as the next iteration's rho)
+          if (!finite_bits(s[0]) || !finite_bits(rho)) {
+            if (!sh.rere || (precon && !finite_bits(rho))) sh.flag |= 2;
+          }
           sh.beta = rho / sh.rho;
           sh.rho = rho;
           ++sh.it;
@@ -330,8 +359,8 @@ __global__ void __launch_bounds__(kST, 2) k_solo_cg(SoloArgs A) {
 template <int OP>
 __global__ void __launch_bounds__(kST, 2) k_solo_bicgstab(SoloArgs A) {
   __shared__ SoloShared sh;
-  SoloGrid grid(A, sh);
-  if (threadIdx.x == 0) sh.lost = 0;
+  SoloGrid<true> grid(A, sh);
+  if (threadIdx.x == 0) sh.lost = sh.huge = 0;
   if (threadIdx.x < 48) sh.conn[threadIdx.x] = A.st.conn[threadIdx.x];
   __syncthreads();
   const size_t n = (size_t)A.n;
@@ -385,13 +414,24 @@ __global__ void __launch_bounds__(kST, 2) k_solo_bicgstab(SoloArgs A) {
       return;
     // x += alpha M p ; r -= alpha v ; M r
     const double alpha = sh.alpha;
+    bool huge = false;
     for (int i = first; i < hi; i += kST) {
       A.x[i] = fma(zp[i], alpha, A.x[i]);
       const double rv = fma(-alpha, v[i], r[i]);
       r[i] = rv;
+      huge |= exponent_field(rv) >= kSoloHuge;
       if (precon) zr[i] = solo_jacobi(A, rv, rd[i], i);
     }
-    if (!grid.sync()) return;
+    if (huge) sh.huge = 1;
+    if (!grid.sync_huge()) return;
+    if (sh.huge) {  // whether ||r||^2 overflows
+      one[0] = 0.0;
+      for (int i = first; i < hi; i += kST) one[0] = fma(r[i], r[i], one[0]);
+      if (!grid.reduce(one, [&](const double (&s)[1]) {
+            if (!finite_bits(s[0])) sh.flag |= 2;
+          }))
+        return;
+    }
     // t = A M r ; omega = t.r / t.t
     two[0] = two[1] = 0.0;
     for (int i = first; i < hi; i += kST) {
@@ -428,7 +468,7 @@ __global__ void __launch_bounds__(kST, 2) k_solo_bicgstab(SoloArgs A) {
       two[1] = fma(rv, rv, two[1]);
     }
     if (!grid.reduce(two, [&](const double (&s)[2]) {
-          if (!finite_bits(s[0]) || !finite_bits(s[1]) || !finite_bits(sh.omega)) sh.flag |= 2;
+          if (!finite_bits(s[0]) || !finite_bits(sh.omega)) sh.flag |= 2;
           if (sh.omega == 0.0 || sh.rho == 0.0) sh.flag |= 1;
           sh.beta = (s[0] / sh.rho) * (sh.alpha / sh.omega);
           sh.rho = s[0];
