@@ -119,6 +119,14 @@ struct BatchShared {
   int item;
 };
 
+// v^2 rounds to more than 0 for |v| above 2^-537.5, whose square is half the smallest
+// double: the largest double below it, and the magnitude's upper half to compare with
+// its upper half first
+constexpr long long kZeroSquare = 0x1e56a09e667f3bccll;
+__device__ __forceinline__ int upper_magnitude(double v) {
+  return __double2hiint(v) & 0x7fffffff;
+}
+
 // in-grid neighbours of row i: bits 0..5 for -d0, +d0, -d1, +d1, -d2, +d2
 __device__ __forceinline__ unsigned row_mask(const BatchSys &S, unsigned i) {
   const unsigned n2 = (unsigned)S.n2, n1 = (unsigned)S.n1, q = i / n2;
@@ -296,15 +304,19 @@ __device__ void solve_system(const BatchArgs &A, int id, BatchShared &shm) {
     });
     if (st.status) break;
     const double alpha = st.alpha;
-    // r -= alpha v; whether ||r||^2 is 0 (no r of 2^-538 or more) by the
-    // exponents, off the FP64 pipe
-    bool live = false;
+    // r -= alpha v; whether ||r||^2 is 0 (no entry's square rounds to more) by the
+    // largest magnitude's bits, off the FP64 pipe
+    int top = 0;
 #pragma unroll 2
     for (unsigned i = first; i < hi; i += kT) {
       const double rv = fma(-alpha, v[i], r[i]);
       r[i] = rv;
-      live |= exponent_field(rv) >= 1023 - 538;
+      top = max(top, upper_magnitude(rv));
     }
+    bool live = top > (int)(kZeroSquare >> 32);
+    if (top == (int)(kZeroSquare >> 32))
+      for (unsigned i = first; i < hi; i += kT)
+        live |= (__double_as_longlong(r[i]) & 0x7fffffffffffffffll) > kZeroSquare;
     team.sync();
     // t = A J(r) ; omega = t.r / t.t
     two[0] = two[1] = 0.0;
@@ -330,11 +342,10 @@ __device__ void solve_system(const BatchArgs &A, int id, BatchShared &shm) {
       if (st.exact) st.res2 = 0.0;
     });
     const double as = st.as;
-    if (st.exact) {
+    if (st.exact || st.status) {  // the iteration ends with the alpha step
       for (unsigned i = first; i < hi; i += kT) x[i] = fma(p[i], as, x[i]);
       break;
     }
-    if (st.status) break;
     // x += alpha J(p) + omega J(r) ; r -= omega t (or r = b - A x) ;
     // rho_new = r.r0, res2 = r.r
     const double omega = st.omega, os = st.os;
