@@ -3072,6 +3072,7 @@ static lgx_status vcycle_impl(lgx_amg &h, const XT *b0, XT *x0, cudaStream_t s) 
 
 lgx_colouring *amg_finest_colouring(lgx_amg &h) { return h.lv[0]->col.get(); }
 const Csr &amg_finest_matrix(const lgx_amg &h) { return *h.lv[0]->a; }
+int amg_outer_config(const lgx_amg &h) { return h.outer_config; }
 
 // Applies the preconditioner in the finest level's permuted space with
 // double vectors (the outer Krylov vectors).

@@ -52,6 +52,8 @@ struct lgx_amg {
   int32_t stop_reason = 0;           // LGX_STOP_* (hierarchy/wright.hpp:26-28)
   lgx::DBuf<double> nat_b, nat_x;    // natural-order staging for lgx_amg_vcycle
   bool f32 = false;
-  bool tuned_outer = false;          // the autotuner set the finest matrix's product slot
+  // the autotuner's configuration for the solves' product with the finest matrix in
+  // natural order (the caller's, whose own choice is its own); -1: none
+  int8_t outer_config = -1;
 };
 

@@ -237,15 +237,18 @@ lgx_status csr_compute_max_window(Csr &a, cudaStream_t s);
 // sets max_row and max_win of `count` matrices from their row offsets
 lgx_status csr_compute_extents(Csr *const *list, int count, cudaStream_t s);
 
-// y = A x for CSR with value type VT and vector type XT (accumulation in XT)
+// y = A x for CSR with value type VT and vector type XT (accumulation in XT);
+// config: the row engine's configuration where the caller has tuned one of its own
+// (-1: the matrix's)
 template <typename VT, typename XT>
-lgx_status csr_spmv(const Csr &a, const VT *val, const XT *x, XT *y, cudaStream_t s);
+lgx_status csr_spmv(const Csr &a, const VT *val, const XT *x, XT *y, cudaStream_t s,
+                    int config = -1);
 // r = b - A x; if norm != nullptr, norm[0] = ||r||^2 (double, deterministic)
 // scale: per-row factor of bfloat16 values (value = scale[row] * stored)
 template <typename VT, typename XT>
 lgx_status csr_residual(const Csr &a, const VT *val, const XT *b, const XT *x, XT *r,
                         double *norm, double *partials, unsigned *counter, cudaStream_t s,
-                        const float *scale = nullptr);
+                        const float *scale = nullptr, int config = -1);
 
 // grid rows without column indices (lgx_grid.cu): each runs when
 // `a` carries a grid mirroring `val` (*done), else leaves the work to the

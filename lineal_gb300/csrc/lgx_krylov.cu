@@ -21,6 +21,7 @@ namespace lgx {
 lgx_status amg_apply_permuted(lgx_amg &h, const double *b, double *x, cudaStream_t s);
 lgx_colouring *amg_finest_colouring(lgx_amg &h);
 const Csr &amg_finest_matrix(const lgx_amg &h);
+int amg_outer_config(const lgx_amg &h);
 bool amg_cycle_f32(const lgx_amg &h);
 lgx_status amg_apply_permuted_f32(lgx_amg &h, const float *b, float *x, cudaStream_t s);
 const float *amg_finest_values_f32(const lgx_amg &h);
@@ -248,6 +249,7 @@ struct Solver {
   const lgx_matrix *m = nullptr;  // natural-order operator (when pcsr == nullptr)
   const Csr *pcsr = nullptr;      // CSR operator in the preconditioner's order
   const int32_t *perm = nullptr;  // that order -> natural; null: natural order
+  int config = -1;                // the hierarchy's tuned configuration for pcsr's products
   int precon = LGX_PRECON_NONE;
   double relax = 1.0;
   int ultra = 0;
@@ -284,8 +286,9 @@ struct Solver {
   }
   lgx_status apply(const double *x, double *y) {
     if (pcsr) {
-      if (pcsr->storage == LGX_F64) return csr_spmv<double, double>(*pcsr, pcsr->v64.p, x, y, s);
-      return csr_spmv<float, double>(*pcsr, pcsr->v32.p, x, y, s);
+      if (pcsr->storage == LGX_F64)
+        return csr_spmv<double, double>(*pcsr, pcsr->v64.p, x, y, s, config);
+      return csr_spmv<float, double>(*pcsr, pcsr->v32.p, x, y, s, config);
     }
     return matrix_spmv(m, x, y, s);
   }
@@ -293,9 +296,9 @@ struct Solver {
     if (pcsr) {
       if (pcsr->storage == LGX_F64)
         return csr_residual<double, double>(*pcsr, pcsr->v64.p, b, x, r, norm, partials.p,
-                                            counters.p, s);
+                                            counters.p, s, nullptr, config);
       return csr_residual<float, double>(*pcsr, pcsr->v32.p, b, x, r, norm, partials.p,
-                                         counters.p, s);
+                                         counters.p, s, nullptr, config);
     }
     return matrix_residual(m, b, x, r, norm, partials.p, counters.p, s);
   }
@@ -412,6 +415,7 @@ static lgx_status setup_solver(const lgx_matrix *a, const lgx_solve_params *p, c
             return fail(LGX_ERR_INVALID, "the hierarchy was built on a stencil matrix");
         } else if (c->natural) {
           S.pcsr = &amg_finest_matrix(*p->amg);  // natural order: the matrix as it is
+          S.config = amg_outer_config(*p->amg);
         } else {
           S.pcsr = &c->pcsr;
           S.perm = c->perm.p;

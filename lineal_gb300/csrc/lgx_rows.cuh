@@ -667,14 +667,16 @@ inline lgx_status launch_spread(int64_t rb, int64_t re, const Csr &a, const VT *
   return LGX_OK;
 }
 
-// rows [rb, re) of `a` (values `val`) through the engine configuration the
-// autotuner chose for this matrix and operation, else the process-wide one
+// rows [rb, re) of `a` (values `val`) through the engine configuration that the
+// caller names, else the one the autotuner chose for this matrix and operation,
+// else the process-wide one
 template <typename VT, class Op>
 inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *val, const Op &op,
-                              cudaStream_t s) {
+                              cudaStream_t s, int config = -1) {
   if (re <= rb) return LGX_OK;
   bool done = false;
-  const int tuned = a.tuned[TuneClass<Op>::value][tune_value_index<VT>()];
+  const int tuned =
+    config >= 0 ? config : a.tuned[TuneClass<Op>::value][tune_value_index<VT>()];
   const int cfg = tuned >= 0 ? tuned : rows_config();
   if constexpr (!Op::kReduce) {  // (a reduction wants few, large CTAs)
     if (cfg == 3 || cfg == 7) {

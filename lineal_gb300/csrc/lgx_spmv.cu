@@ -63,31 +63,32 @@ struct ResidualOp {
 };
 
 template <typename VT, typename XT>
-lgx_status csr_spmv(const Csr &a, const VT *val, const XT *x, XT *y, cudaStream_t s) {
+lgx_status csr_spmv(const Csr &a, const VT *val, const XT *x, XT *y, cudaStream_t s, int config) {
   if (a.n == 0) return LGX_OK;
   bool done = false;
   LGX_CHECK((grid_spmv<VT, XT>(a, val, x, y, s, &done)));
   if (done) return LGX_OK;
-  return launch_rows<VT>(0, a.n, a, val, SpmvOp<VT, XT>{x, y}, s);
+  return launch_rows<VT>(0, a.n, a, val, SpmvOp<VT, XT>{x, y}, s, config);
 }
 
 template <typename VT, typename XT>
 lgx_status csr_residual(const Csr &a, const VT *val, const XT *b, const XT *x, XT *r,
                         double *norm, double *partials, unsigned *counter, cudaStream_t s,
-                        const float *scale) {
+                        const float *scale, int config) {
   if (a.n == 0) {
     if (norm) LGX_CUDA(cudaMemsetAsync(norm, 0, sizeof(double), s));
     return LGX_OK;
   }
   if (norm)
     return launch_rows<VT>(0, a.n, a, val,
-                           ResidualOp<VT, XT, true>{b, x, r, norm, partials, counter, scale}, s);
+                           ResidualOp<VT, XT, true>{b, x, r, norm, partials, counter, scale}, s,
+                           config);
   bool done = false;
   LGX_CHECK((grid_residual<VT, XT>(a, val, b, x, r, scale, s, &done)));
   if (done) return LGX_OK;
   return launch_rows<VT>(0, a.n, a, val,
-                         ResidualOp<VT, XT, false>{b, x, r, nullptr, nullptr, nullptr, scale},
-                         s);
+                         ResidualOp<VT, XT, false>{b, x, r, nullptr, nullptr, nullptr, scale}, s,
+                         config);
 }
 
 // partial-sum slots of a reducing row launch
@@ -95,23 +96,23 @@ lgx_status csr_residual(const Csr &a, const VT *val, const XT *b, const XT *x, X
 int64_t csr_partials(int64_t /*n*/) { return (int64_t)sm_count() * kRowsMaxCtasPerSm; }
 
 template lgx_status csr_spmv<double, double>(const Csr &, const double *, const double *,
-                                             double *, cudaStream_t);
+                                             double *, cudaStream_t, int);
 template lgx_status csr_spmv<float, double>(const Csr &, const float *, const double *, double *,
-                                            cudaStream_t);
+                                            cudaStream_t, int);
 template lgx_status csr_spmv<float, float>(const Csr &, const float *, const float *, float *,
-                                           cudaStream_t);
+                                           cudaStream_t, int);
 template lgx_status csr_residual<double, double>(const Csr &, const double *, const double *,
                                                  const double *, double *, double *, double *,
-                                                 unsigned *, cudaStream_t, const float *);
+                                                 unsigned *, cudaStream_t, const float *, int);
 template lgx_status csr_residual<float, double>(const Csr &, const float *, const double *,
                                                 const double *, double *, double *, double *,
-                                                unsigned *, cudaStream_t, const float *);
+                                                unsigned *, cudaStream_t, const float *, int);
 template lgx_status csr_residual<float, float>(const Csr &, const float *, const float *,
                                                const float *, float *, double *, double *,
-                                               unsigned *, cudaStream_t, const float *);
+                                               unsigned *, cudaStream_t, const float *, int);
 template lgx_status csr_residual<bf16, float>(const Csr &, const bf16 *, const float *,
                                               const float *, float *, double *, double *,
-                                              unsigned *, cudaStream_t, const float *);
+                                              unsigned *, cudaStream_t, const float *, int);
 
 // ---------------------------------------------------------------------------
 // Matrix-free 7-point diffusion stencil

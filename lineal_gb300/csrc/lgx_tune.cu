@@ -260,16 +260,17 @@ lgx_status tune_level(lgx_colouring &c, const VT *val, const float *scale, doubl
   return LGX_OK;
 }
 
-// y = A x with FP64 vectors (the outer Krylov product and lgx_spmv)
-lgx_status tune_product64(Csr &a, int level, int reps, cudaStream_t s,
+// y = A x with FP64 vectors (the outer Krylov product and lgx_spmv); the choice
+// goes to `slot`
+lgx_status tune_product64(const Csr &a, int8_t &slot, int level, int reps, cudaStream_t s,
                           std::vector<lgx_tune_entry> &out) {
   Scratch<double> v;
   LGX_CHECK(v.alloc(a.n, s));
   const bool f64 = a.storage == LGX_F64;
   lgx_tune_entry e = blank_entry(level, 0, f64 ? 8 : 4);
-  LGX_CHECK(tune_slot(a.tuned[0][f64 ? 0 : 1], reps, s, e, [&](cudaStream_t cs) {
-    return f64 ? csr_spmv<double, double>(a, a.v64.p, v.x.p, v.r.p, cs)
-               : csr_spmv<float, double>(a, a.v32.p, v.x.p, v.r.p, cs);
+  LGX_CHECK(tune_slot(slot, reps, s, e, [&](cudaStream_t cs) {
+    return f64 ? csr_spmv<double, double>(a, a.v64.p, v.x.p, v.r.p, cs, slot)
+               : csr_spmv<float, double>(a, a.v32.p, v.x.p, v.r.p, cs, slot);
   }));
   out.push_back(e);
   return LGX_OK;
@@ -293,7 +294,9 @@ lgx_status lgx_matrix_autotune(lgx_matrix *a, int reps, lgx_tune_entry *out, lgx
   if (a->kind != LGX_MATRIX_CSR) return fail(LGX_ERR_UNSUPPORTED, "autotune needs a CSR matrix");
   if (reps < 1 || reps > 1000) return fail(LGX_ERR_INVALID, "reps must be in [1, 1000]");
   std::vector<lgx_tune_entry> all;
-  if (a->csr.n > 0) LGX_CHECK(tune_product64(a->csr, 0, reps, (cudaStream_t)stream, all));
+  if (a->csr.n > 0)
+    LGX_CHECK(tune_product64(a->csr, a->csr.tuned[0][a->csr.storage == LGX_F64 ? 0 : 1], 0, reps,
+                             (cudaStream_t)stream, all));
   else all.push_back(blank_entry(0, 0, a->csr.storage == LGX_F64 ? 8 : 4));
   return copy_out(all, out, 1, nullptr);
 }
@@ -315,16 +318,10 @@ lgx_status lgx_amg_autotune(lgx_amg *h, int reps, lgx_tune_entry *out, int max_o
     if (!lv.col || l == L - 1 || lv.col->pcsr.n == 0 || lv.col->pcsr.grid) continue;
     lgx_colouring &c = *lv.col;
     if (l == 0 && lv.a->storage == LGX_F64 && h->f32) {
-      if (!c.natural) {
-        LGX_CHECK(tune_product64(c.pcsr, 0, reps, s, all));
-      } else {
-        // the caller's matrix itself: a choice it already made stays
-        Csr &a = const_cast<Csr &>(*lv.a);
-        const int8_t own = h->tuned_outer ? (int8_t)-1 : a.tuned[0][0];
-        LGX_CHECK(tune_product64(a, 0, reps, s, all));
-        if (own >= 0) a.tuned[0][0] = own;
-        else h->tuned_outer = true;
-      }
+      // in natural order the solves multiply by the caller's matrix, which other
+      // hierarchies and threads use too: the choice stays here
+      LGX_CHECK(tune_product64(c.natural ? *lv.a : c.pcsr,
+                               c.natural ? h->outer_config : c.pcsr.tuned[0][0], 0, reps, s, all));
     }
     if (!h->f32) {
       if (c.pcsr.storage == LGX_F64)
@@ -351,9 +348,6 @@ lgx_status lgx_amg_autotune_reset(lgx_amg *h) {
     if (lv->col)
       for (int op = 0; op < 2; ++op)
         for (int vi = 0; vi < 3; ++vi) set_slot(*lv->col, op, vi, -1);
-  if (h->tuned_outer) {
-    const_cast<Csr &>(*h->lv[0]->a).tuned[0][0] = -1;
-    h->tuned_outer = false;
-  }
+  h->outer_config = -1;
   return LGX_OK;
 }
