@@ -697,8 +697,10 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
   // rows read hundreds of lines, and a row has fewer rounds.  AMG-CG at 256^3,
   // 27 points, FP64: 429 -> 419 ms; float vectors, 121 x 117 x 125, 27 points:
   // 64.3 -> 57.0; shorter rows (256^3, 7 points) the same or slower (290 / 292).
+  // (Part of configuration 3, like the forms for few tiles and short rows above,
+  // whether it is the process-wide one or the autotuner's.)
   if constexpr (StagedForm<Op>::value && TuneClass<Op>::value == 1) {
-    if (tuned < 0 && cfg == 3 && op.spread() && a.nnz > Op::kLongRow * a.n)
+    if (cfg == 3 && op.spread() && a.nnz > Op::kLongRow * a.n)
       LGX_CHECK((launch_wrows<VT, Op, 8, 1>(rb, re, a, val, op, s, &done)));
     if (done) return LGX_OK;
   }

@@ -1,5 +1,8 @@
 """What the autotuner's choices reach, by the names of the kernels that run: a
-hierarchy's choice for its finest product stays with that hierarchy."""
+hierarchy's choice for its finest product stays with that hierarchy, and a level
+that is tuned to the process-wide configuration runs what an untuned one runs."""
+
+import re
 
 import numpy as np
 import pytest
@@ -69,3 +72,20 @@ def test_product_choice_stays_with_its_hierarchy(cuda, records):
         assert solve(h) == solve(other) == set(own)
     finally:
         cuda.row_engine(before)
+
+
+def test_default_choice_runs_the_default(cuda, records):
+    """The tuner times the process-wide configuration (3) as it runs untuned: the
+    first warp-tile launches of the finest level's sweeps are the untuned ones
+    (1.06M rows of 27 entries: more than eight tiles per SM and colour)."""
+    assert cuda.row_engine() == 3
+    dims = (101, 102, 103)
+    m = _matrix(cuda, dims)
+    h = cuda.HierarchyWright(**PARAMS).instantiate(m)
+    b = np.random.default_rng(2).uniform(-1, 1, m.row_num())
+    shape = lambda names: [re.search(r"k_wrows<.*>", k).group() for k in names
+                           if "k_wrows<" in k and "lgx::SorOp<double, double>" in k]
+    # the last backward sweep of a cycle is the finest level's
+    untuned = shape(_kernels(lambda: h.vcycle(b)))[-2]
+    tuned = shape(_kernels(lambda: h.autotune(reps=1)))
+    assert tuned[0] == untuned
