@@ -591,9 +591,13 @@ lgx_status colouring_build_natural(const Csr &a, const int32_t *d_colour, int32_
     LGX_CHECK(csr_alloc_arrays(*list[k], nnz[k], storage));
   }
   if (n == 0) return LGX_OK;
+  // (0 stands where a row stored no diagonal, as k_colour_rdiag has it: such a row
+  // divides by 0.  Matrices without one are refused where they are created.)
   LGX_CHECK(out.pdiag.alloc(n));
+  LGX_CUDA(cudaMemsetAsync(out.pdiag.p, 0, sizeof(double) * (size_t)n, s));
   if (storage == LGX_F64) {
     LGX_CHECK(out.rdiag.alloc(n));
+    LGX_CUDA(cudaMemsetAsync(out.rdiag.p, 0, sizeof(double) * (size_t)n, s));
     k_half_fill<double, double><<<g, 256, 0, s>>>(
       n, a.rowptr.p, a.col.p, a.v64.p, out.perm.p, out.colour.p, rows_out<double>(out.pcsr),
       rows_out<double>(out.lo), rows_out<double>(out.up), out.pdiag.p, out.rdiag.p);
