@@ -2657,6 +2657,31 @@ static lgx_status colouring_smallest_last(const Csr &a, cudaStream_t s, DBuf<int
   return LGX_OK;
 }
 
+// Whether the levels in natural order leave enough memory.  Their rows and halves
+// hold every entry twice (24 bytes in FP64, 16 in float, where colour order takes 12
+// and 16 or, of a float matrix, 8): 27 points, 100^3, FP64, the set-up needs 36
+// bytes per finest entry of free memory instead of 21.  They may take a third of
+// what is free; the other two thirds hold what follows (transfers, cycle vectors,
+// and with 7 entries a row still 40 vectors of a solve), so that a system which
+// is set up and solved in colour order is not refused for its speed.
+static bool natural_fits(const lgx_amg &h, bool given_finest) {
+  int64_t bytes = 0;
+  for (size_t l = given_finest ? 1 : 0; l + 1 < h.lv.size(); ++l) {
+    const lgx_amg_level &lv = *h.lv[l];
+    if (lv.stencil) continue;
+    const Csr &a = *lv.a;
+    const bool f64 = a.storage == LGX_F64;
+    bytes += 2 * a.nnz * (h.f32 || !f64 ? 8 : 12) + 40 * a.n;
+    if (l == 0 && h.f32 && f64) bytes += 4 * a.nnz;
+  }
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return bytes <= (int64_t)(free_bytes / 3);
+}
+
 static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
                             const lgx_colouring *finest_colouring, const lgx_agg_map *maps,
                             int64_t nmaps, cudaStream_t s, lgx_amg &h) {
@@ -2742,6 +2767,7 @@ static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
     if (stop) break;
   }
   const int64_t L = (int64_t)h.lv.size();
+  const bool room = natural_fits(h, finest_colouring != nullptr);
   // smoother colourings (all but the coarsest level)
   for (int64_t l = 0; l + 1 < L; ++l) {
     lgx_amg_level &lv = *h.lv[l];
@@ -2774,8 +2800,8 @@ static lgx_status amg_build(const lgx_matrix *m, const lgx_amg_params &p,
     // 121 x 117 x 125, 27 points, 73 -> 67; FP64 at 256^3, 27 points, 535 ->
     // 501.  A given finest
     // colouring keeps colour order, which is the order its grid kernels need;
-    // bfloat16 values keep it too.
-    const bool natural = !(l == 0 && finest_colouring) && !(h.f32 && p.cycle_bf16);
+    // bfloat16 values keep it too, and all levels where memory is short.
+    const bool natural = room && !(l == 0 && finest_colouring) && !(h.f32 && p.cycle_bf16);
     if (l == 0 && finest_colouring) {
       LGX_CHECK(colouring_build(*lv.a, finest_colouring->colour.p, finest_colouring->ncolours, s,
                                 *lv.col));
