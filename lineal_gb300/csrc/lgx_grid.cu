@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <cstring>
 
 #include "lgx_internal.cuh"
 #include "lgx_rows.cuh"
@@ -851,19 +852,22 @@ static const CUtensorMap *g27_value_map(const Grid27 &gr, const T *v) {
   return map;
 }
 
-// the boxes of k_g27_vhalf on the float values (null: no tensor maps)
-static bool g27_half_maps(const Grid27 &gr, const float *v, GHalfMaps *out) {
+// the boxes of k_g27_vhalf on the float values, where its launches can use them
+static bool g27_half_maps(Grid27 &gr) {
   const G27EncodeFn encode = g27_encode();
-  if (!encode) return false;
+  if (!encode || !gr.v32.p || (gr.stride * (int64_t)sizeof(float)) % 16 != 0 ||
+      gr.stride > (int64_t)INT32_MAX)
+    return false;
+  static_assert(sizeof(CUtensorMap) == sizeof(gr.hmap32[0]), "tensor map storage");
   const cuuint64_t gdim[2] = {(cuuint64_t)gr.stride, (cuuint64_t)gr.points};
   const cuuint64_t gstride[1] = {(cuuint64_t)gr.stride * sizeof(float)};
   const cuuint32_t estride[2] = {1, 1};
   const int high[3] = {gr.points == 27 ? 9 : 7, 3, 1};
   for (int k = 0; k < 3; ++k) {
     const cuuint32_t box[2] = {(cuuint32_t)g_rows_per_cta<float>(), (cuuint32_t)high[k]};
-    if (encode(&out->m[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(v), gdim,
-               gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    if (encode(reinterpret_cast<CUtensorMap *>(gr.hmap32[k]), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+               gr.v32.p, gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return false;
   }
@@ -876,10 +880,10 @@ static lgx_status launch_half_pts(const Grid27 &gr, const VT *v, int64_t rb, int
                                   const XT *b, XT *x, XT *y, const G27Sor &so, cudaStream_t s) {
   const bool pdl = sizeof(XT) == 4 || re - rb <= pdl_fp64_rows();
   if constexpr (std::is_same_v<VT, float> && std::is_same_v<XT, float>) {
-    GHalfMaps maps;
-    if (g27_tma_enabled() && rb % 4 == 0 && ((uintptr_t)v & 15u) == 0 &&
-        (gr.stride * (int64_t)sizeof(float)) % 16 == 0 && gr.stride <= (int64_t)INT32_MAX &&
-        g27_half_maps(gr, v, &maps)) {
+    // (v is gr.v32, see grid_values; rows in fours start on 16 bytes)
+    if (g27_tma_enabled() && rb % 4 == 0 && gr.half_maps) {
+      GHalfMaps maps;
+      std::memcpy(maps.m, gr.hmap32, sizeof(maps.m));
       constexpr int RT = g_rows_per_cta<float>();
       LGX_CUDA(launch_pdl(pdl, k_g27_vhalf<UP, PTS>, dim3((unsigned)((re - rb + RT - 1) / RT)),
                           dim3(RT), 0, s, maps, view(gr), rb, re, b, x, y, so,
@@ -1205,6 +1209,7 @@ lgx_status grid27_attach(lgx_colouring &c, const int64_t dims[3], int points, cu
   LGX_CUDA(cudaMemcpyAsync(&h_bad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   LGX_CUDA(cudaStreamSynchronize(s));
   if (h_bad) return LGX_OK;  // not this structure: the CSR path stays
+  gr->half_maps = g27_half_maps(*gr);
   c.pcsr.grid = gr;
   *attached = true;
   return LGX_OK;

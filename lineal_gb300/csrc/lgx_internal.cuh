@@ -145,6 +145,10 @@ struct Grid27 {
   alignas(64) mutable unsigned char vmap32[128] = {};
   alignas(64) mutable unsigned char vmap64[128] = {};
   mutable const void *vmap32_key = nullptr, *vmap64_key = nullptr;
+  // the float values in boxes of 9, 3 and 1 planes (7 points: 7, 3, 1), for the
+  // half rows; encoded when the grid is attached (false: no tensor maps)
+  alignas(64) unsigned char hmap32[3][128] = {};
+  bool half_maps = false;
 };
 
 // Csr::tuned index of a value type
