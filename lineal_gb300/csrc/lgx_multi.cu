@@ -1,9 +1,10 @@
 // Multi-right-hand-side (blocked) AMG-PCG: up to 32 right-hand sides share
-// every pass over the matrices.  Vectors are row-major blocks, X[i * K + k],
-// and in every kernel lane k of a warp handles column k: a row's column
-// indices and values are read once (one coalesced load of up to 32 entries,
-// then broadcast by shuffles) and applied to all K columns, whose gathers
-// x[c * K + k] are contiguous.  Per column the arithmetic is the
+// every pass over the matrices.  Vectors are row-major blocks, X[i * K + k].  In
+// the row kernels a group of lanes shares a row, a few columns per lane (MLane),
+// and a row's column indices and values are read once by the group (a lane an
+// entry, then broadcast by shuffles) and applied to all K columns, whose gathers
+// x[c * K + k] are contiguous; in the dots and the dense solve lane k of a warp
+// handles column k.  Per column the arithmetic is the
 // single-vector one (products in storage order, SOR row formula, aggregate
 // sums in list order), so each column follows its own CG recurrence; the CG
 // scalars are per column and a converged column is frozen.
@@ -498,7 +499,7 @@ static lgx_status m_level_sor(const lgx_amg &h, const lgx_amg_level &lv, int K, 
 
 // With relax 1 the residual that follows a forward sweep from zero is 0 in the
 // rows of the last colour (mc_up_residual): permuted levels compute the rows
-// before m_zero_from only, the others stay 0 from the start.
+// before m_zero_from only, and the restriction does not read the others.
 static int64_t m_zero_from(const lgx_amg &h, const lgx_amg_level &lv) {
   const lgx_colouring &c = *lv.col;
   if (c.natural || h.p.smoother_relax != 1.0 || h.p.smoother_ultra || c.ncolours < 1)
@@ -744,12 +745,6 @@ static lgx_status pcg_multi(const lgx_matrix *a, lgx_amg &h, int K, const double
       LGX_CHECK(w.b[l].alloc(nl));
       LGX_CHECK(w.x[l].alloc(nl));
     }
-  }
-  if (L > 1) {
-    // (the last colour's rows of a permuted finest level: see m_zero_from)
-    const int64_t z0 = std::min(m_zero_from(h, *h.lv[0]), n);
-    if (z0 < n)
-      LGX_CUDA(cudaMemsetAsync(w.r[0].p + z0 * K, 0, sizeof(XT) * (size_t)((n - z0) * K), s));
   }
   // A float cycle reads R as float (w.b[0], written by k_mupdate or converted)
   // and leaves Z as float in w.x[0], which the dots and the direction read.
