@@ -58,8 +58,10 @@ enum Post {
 };
 
 // whether the update that follows a direction must not take place: its rho is
-// zero or a flag is up, so the host will stop at the iteration before it.
-// Nothing but p, q and z changes from then on.
+// zero or a flag is up, so the host will stop at the iteration before it.  From
+// then on x stays as it is; p, q and z change, and an iteration that recomputes the
+// residual writes r and res2 again, for the same x.  The host takes the norm it
+// reports before it sees the halt, and reads no more than the flags after it.
 __device__ __forceinline__ bool gate(KScalars *ks, int post) {
   if (post == POST_ALPHA_GATED && (ks->flag || ks->rho == 0.0)) {
     ks->halt = 1;
@@ -720,7 +722,7 @@ static lgx_status run_overlapped(lgx_krylov &K, double &res, double *history) {
     st = check_flags(K.h, K.it);
     if (st != LGX_OK) break;
   }
-  LGX_CHECK(K.S.read(K.h));
+  LGX_CHECK(K.S.read(K.h));  // (for its flags; res belongs to iteration K.it, see gate)
   return st != LGX_OK ? st : check_flags(K.h, K.it);
 }
 

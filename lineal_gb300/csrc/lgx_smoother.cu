@@ -2,9 +2,14 @@
 // the GB300 replacement of the thread-block-hybrid SOR of
 // gauss-seidel-variant/sweep.hpp:134-200, plus graph colouring.
 //
-// A multicolour sweep works on a colour-permuted copy of the matrix: colour c
-// occupies the contiguous rows [offsets[c], offsets[c+1]), so every colour
-// pass is a coalesced row-block kernel.  Rows keep their original column
+// A multicolour sweep works on a copy of the matrix with its rows in colour order:
+// colour c occupies the contiguous rows [offsets[c], offsets[c+1]), so every colour
+// pass is a coalesced row-block kernel.  In the colour-permuted form (a colouring
+// by itself, a hierarchy's finest level with a given colouring) the columns and the
+// vectors are in that order too; in the natural-order form (the other levels of a
+// hierarchy, lgx_colouring::natural) columns and vectors stay as they are, a list
+// names the vector row of each matrix row, and sweeps from zero and the residuals
+// after them run on halves of the rows.  Either way rows keep their original column
 // order, hence each row sum is formed in exactly the order of the
 // reference's scalar CSR path; the sweep equals the reference SOR run in the
 // order "rows sorted by (colour, index)".

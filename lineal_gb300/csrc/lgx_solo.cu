@@ -4,7 +4,8 @@
 // On systems that fit the L2 an iteration is a few microseconds of work behind
 // five to eight launches and a host round trip: 52 us per Jacobi-CG iteration on
 // the 64^3 lookup stencil, of which its FP64 operations take 7.  Here one CTA
-// per SM or two keep the vectors' slices, the phases of
+// per SM or two own a slice of the rows each (their vectors stay in a workspace in
+// global memory, which the L2 holds), the phases of
 // conjugate-gradients/solver.hpp:75-115 and bicgstab/solver.hpp:73-151 are
 // separated by grid barriers, every CTA adds the same partial sums in the same
 // order (so all take the same decisions) and the stopping rule of
