@@ -3443,6 +3443,12 @@ lgx_status lgx_amg_vcycle(lgx_amg *h, const double *d_b, double *d_x, lgx_stream
     LGX_CHECK(amg_apply_permuted(*h, h->nat_b.p, h->nat_x.p, stream));
     return scatter<double, double>(n, perm, h->nat_x.p, d_x, stream);
   }
+  if (overlap(d_b, d_x, sizeof(double) * (size_t)n)) {
+    // the cycle reads b until its end
+    LGX_CUDA(cudaMemcpyAsync(h->nat_b.p, d_b, sizeof(double) * (size_t)n,
+                             cudaMemcpyDeviceToDevice, stream));
+    d_b = h->nat_b.p;
+  }
   return amg_apply_permuted(*h, d_b, d_x, stream);
 }
 

@@ -94,6 +94,12 @@ struct DBuf {
   }
 };
 
+// whether two arrays of `bytes` bytes share memory
+inline bool overlap(const void *a, const void *b, size_t bytes) {
+  const char *p = (const char *)a, *q = (const char *)b;
+  return p < q + bytes && q < p + bytes;
+}
+
 constexpr uint32_t kUnaggregated = 0xFFFFFFFFu;
 // trailing elements of every CSR column/value buffer (the staged row kernels
 // copy 16-byte-aligned spans that may reach past the last entry)

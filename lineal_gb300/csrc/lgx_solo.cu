@@ -503,11 +503,6 @@ lgx_status solo_kernel(bool cg, int64_t n, void **fn, int *most) {
   return LGX_OK;
 }
 
-bool overlap(const void *a, const void *b, size_t bytes) {
-  const char *p = (const char *)a, *q = (const char *)b;
-  return p < q + bytes && q < p + bytes;
-}
-
 }  // namespace
 
 // Runs the solve when the system is one for this path (*done), else leaves it.
