@@ -147,6 +147,28 @@ __device__ __forceinline__ void issue_tile(const int64_t *rowptr, const int32_t 
   if (vb) bulk_g2s(st.val, val + v0, vb, bar);
 }
 
+// autotuner slot of an operation: Op::kTuneClass when declared (SOR sweeps
+// declare 1), else 0 (products)
+template <class Op, class = void>
+struct TuneClass {
+  static constexpr int value = 0;
+};
+template <class Op>
+struct TuneClass<Op, std::void_t<decltype(Op::kTuneClass)>> {
+  static constexpr int value = Op::kTuneClass;
+};
+
+// whether an operation's rows run in rounds of W gathers; the others (kRounds =
+// false) walk their entries one by one
+template <class Op, class = void>
+struct Rounds {
+  static constexpr bool value = true;
+};
+template <class Op>
+struct Rounds<Op, std::enable_if_t<!Op::kRounds>> {
+  static constexpr bool value = false;
+};
+
 // whether an operation names the vector rows of its matrix rows in a list
 template <class Op, class = void>
 struct RowList {
@@ -179,6 +201,7 @@ __device__ __forceinline__ double run_row(const Op &op, int64_t r, int32_t i, co
 //     gathers are issued together; FLAT: products without branches, row_dot)
 //   static constexpr bool kList;  const int32_t *rows;  (kList: matrix row r is
 //     vector row rows[r], r itself when rows is null; row() takes both)
+//   static constexpr bool kRounds;  (false: the row walks its entries one by one)
 //   static constexpr bool kReduce;  __device__ void finish(double total) const;
 //   double *partials; unsigned *counter;  (when kReduce)
 template <typename VT, class Op, int KIND>
@@ -527,18 +550,19 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
 int rows_config();
 
 // Whether a row launch carries the programmatic-dependent-launch attribute.
-// Float rows do; FP64 rows up to pdl_fp64_rows(), except launches of long
+// Float rows do; FP64 rows up to pdl_fp64_rows(), except launches in rounds of long
 // rows (over 16 entries on average) in more tiles than SMs: their warps fill
 // the FP64 pipe, and an early-scheduled successor takes the SMs that the
 // running launch left free, so that its own warps pile up there.  27-point
 // colour launches, FP64, with / without: 3.7k rows 4.1 / 4.7 us, 6.9k 5.5 /
 // 4.8, 10.8k 6.1 / 5.1, 16k 6.5 / 6.1; 7-point 5.5k rows 2.4 / 3.3 us, 18k
 // 3.2 / 3.5, 167k 9.8 / 10.8.
-template <typename XT>
+template <class Op>
 inline bool rows_pdl(int64_t rb, int64_t re, const Csr &a) {
-  if (sizeof(XT) == 4) return true;
-  return re - rb <= pdl_fp64_rows() &&
-         (a.nnz <= 16 * a.n || re - rb <= (int64_t)sm_count() * kWarpTileRows);
+  if (sizeof(typename Op::X) == 4) return true;
+  if (re - rb > pdl_fp64_rows()) return false;
+  return !Rounds<Op>::value || a.nnz <= 16 * a.n ||
+         re - rb <= (int64_t)sm_count() * kWarpTileRows;
 }
 
 template <typename VT, class Op, int WPC, int S, int MB = 0>
@@ -573,7 +597,7 @@ inline lgx_status launch_wrows(int64_t rb, int64_t re, const Csr &a, const VT *v
   const int64_t need = (tiles + WPC - 1) / WPC;
   const int64_t g = (int64_t)sm_count() * per_sm;
   const unsigned grid = (unsigned)(need < g ? (need > 0 ? need : 1) : g);
-  const bool pdl = rows_pdl<typename Op::X>(rb, re, a);
+  const bool pdl = rows_pdl<Op>(rb, re, a);
   LGX_CUDA(launch_pdl(pdl, k_wrows<VT, Op, WPC, S, MB>, dim3(grid),
                       dim3(WPC * 32), smem, s, rb, re, capw,
                       (const int64_t *)a.rowptr.p, (const int32_t *)a.col.p, val, op,
@@ -603,17 +627,6 @@ inline lgx_status launch_rows_cfg(int64_t rb, int64_t re, int64_t max_row, const
   count_launch();
   return LGX_OK;
 }
-
-// autotuner slot of an operation: Op::kTuneClass when declared (SOR sweeps
-// declare 1), else 0 (products)
-template <class Op, class = void>
-struct TuneClass {
-  static constexpr int value = 0;
-};
-template <class Op>
-struct TuneClass<Op, std::void_t<decltype(Op::kTuneClass)>> {
-  static constexpr int value = Op::kTuneClass;
-};
 
 // Launches of few tiles (the colours of small levels) in one-warp CTAs: the
 // warps spread evenly over the SMs, and with the rows' whole length in one or
@@ -678,7 +691,10 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
   const int tuned =
     config >= 0 ? config : a.tuned[TuneClass<Op>::value][tune_value_index<VT>()];
   const int cfg = tuned >= 0 ? tuned : rows_config();
-  if constexpr (!Op::kReduce) {  // (a reduction wants few, large CTAs)
+  // (a reduction wants few, large CTAs; rows that walk entry by entry gain nothing
+  // from the small ones: Jacobi sweep, 27 points, four-warp / one-warp CTAs, 13.8k
+  // rows 6.4 / 6.8 us, 32.7k 6.7 / 7.3)
+  if constexpr (!Op::kReduce && Rounds<Op>::value) {
     if (cfg == 3 || cfg == 7) {
       LGX_CHECK((launch_spread<VT, Op>(rb, re, a, val, op, s, &done)));
       if (!done) LGX_CHECK((launch_small<VT, Op>(rb, re, a, val, op, s, &done)));
@@ -687,7 +703,7 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
   }
   // rows of at most 8 entries (7-point operators) at 256^3: FP64 product 350
   // -> 274, float 295 -> 245 us
-  if (TuneClass<Op>::value == 0 && cfg == 3 && a.max_row <= 8) {
+  if (Rounds<Op>::value && TuneClass<Op>::value == 0 && cfg == 3 && a.max_row <= 8) {
     LGX_CHECK((launch_wrows<VT, Op, 4, 1, kShortMb>(rb, re, a, val, op, s, &done)));
     if (done) return LGX_OK;
   }

@@ -34,6 +34,7 @@ struct JacobiOp {
   double relax, m1;
   using X = double;
   static constexpr bool kReduce = false;
+  static constexpr bool kRounds = false;
   double *partials = nullptr;
   unsigned *counter = nullptr;
   template <int W, bool FLAT>
