@@ -550,19 +550,25 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
 int rows_config();
 
 // Whether a row launch carries the programmatic-dependent-launch attribute.
-// Float rows do; FP64 rows up to pdl_fp64_rows(), except launches in rounds of long
-// rows (over 16 entries on average) in more tiles than SMs: their warps fill
-// the FP64 pipe, and an early-scheduled successor takes the SMs that the
-// running launch left free, so that its own warps pile up there.  27-point
-// colour launches, FP64, with / without: 3.7k rows 4.1 / 4.7 us, 6.9k 5.5 /
-// 4.8, 10.8k 6.1 / 5.1, 16k 6.5 / 6.1; 7-point 5.5k rows 2.4 / 3.3 us, 18k
-// 3.2 / 3.5, 167k 9.8 / 10.8.
-template <class Op>
+// Float rows do; FP64 rows up to pdl_fp64_rows(), except some launches of long rows
+// (over 16 entries on average): their warps fill the FP64 pipe, and an
+// early-scheduled successor takes the SMs that the running launch left free, so that
+// its own warps pile up there.  27 points, with / without, us:
+//  - sweeps in more tiles than SMs go without: colour launches of 3.7k rows 4.1 /
+//    4.7, 6.9k 5.5 / 4.8, 10.8k 6.1 / 5.1, 16k 6.5 / 6.1 (7 points 5.5k rows 2.4 /
+//    3.3, 18k 3.2 / 3.5, 167k 9.8 / 10.8);
+//  - products in one-warp CTAs beyond five tiles per SM go without: 7.2k rows 2.65 /
+//    3.57, 13.8k 2.78 / 3.78, 32.7k 5.44 / 4.51 (float values 10.7 / 6.5);
+//  - products in larger CTAs keep it: 69k rows 6.83 / 7.24, 91k 7.15 / 8.61, 185k
+//    13.0 / 14.6 (127k 12.2 / 11.1).
+template <class Op, int WPC>
 inline bool rows_pdl(int64_t rb, int64_t re, const Csr &a) {
   if (sizeof(typename Op::X) == 4) return true;
   if (re - rb > pdl_fp64_rows()) return false;
-  return !Rounds<Op>::value || a.nnz <= 16 * a.n ||
-         re - rb <= (int64_t)sm_count() * kWarpTileRows;
+  if (!Rounds<Op>::value || a.nnz <= 16 * a.n) return true;
+  const int64_t tile_per_sm = (int64_t)sm_count() * kWarpTileRows;
+  if (TuneClass<Op>::value == 1) return re - rb <= tile_per_sm;
+  return WPC > 1 || re - rb <= 5 * tile_per_sm;
 }
 
 template <typename VT, class Op, int WPC, int S, int MB = 0>
@@ -597,7 +603,7 @@ inline lgx_status launch_wrows(int64_t rb, int64_t re, const Csr &a, const VT *v
   const int64_t need = (tiles + WPC - 1) / WPC;
   const int64_t g = (int64_t)sm_count() * per_sm;
   const unsigned grid = (unsigned)(need < g ? (need > 0 ? need : 1) : g);
-  const bool pdl = rows_pdl<Op>(rb, re, a);
+  const bool pdl = rows_pdl<Op, WPC>(rb, re, a);
   LGX_CUDA(launch_pdl(pdl, k_wrows<VT, Op, WPC, S, MB>, dim3(grid),
                       dim3(WPC * 32), smem, s, rb, re, capw,
                       (const int64_t *)a.rowptr.p, (const int32_t *)a.col.p, val, op,
@@ -636,12 +642,15 @@ inline lgx_status launch_rows_cfg(int64_t rb, int64_t re, int64_t max_row, const
 // one-warp CTAs: 27-point FP64 3.7k rows 5.1 / 4.1 us, 16k 9.3 / 6.5, 28k
 // 10.7 / 9.6 (float 3.3 / 2.8, 4.3 / 3.7, 4.9 / 4.3), 55k 12.0 / 12.6 (float
 // 5.3 / 5.6); 7-point float 5.5k rows 2.0 / 1.8 us, 37k 2.4 / 2.2, 167k 5.2 /
-// 5.2.
+// 5.2.  Float products of short rows only up to two tiles per SM (7 points, 7.2k
+// rows 1.54 / 1.45 us, 13.8k 1.49 / 1.54, 32.7k 1.63 / 1.85).
 template <typename VT, class Op>
 inline lgx_status launch_small(int64_t rb, int64_t re, const Csr &a, const VT *val, const Op &op,
                                cudaStream_t s, bool *done) {
-  if (re - rb > (int64_t)sm_count() * 8 * kWarpTileRows) return LGX_OK;
-  if (a.max_row <= 8) return launch_wrows<VT, Op, 1, 1, kSmallMb8>(rb, re, a, val, op, s, done);
+  const bool short_rows = a.max_row <= 8, flt = sizeof(typename Op::X) == 4;
+  const int64_t most = TuneClass<Op>::value == 0 && short_rows && flt ? 2 : 8;
+  if (re - rb > (int64_t)sm_count() * most * kWarpTileRows) return LGX_OK;
+  if (short_rows) return launch_wrows<VT, Op, 1, 1, kSmallMb8>(rb, re, a, val, op, s, done);
   if (a.max_row <= 16)
     return launch_wrows<VT, Op, 1, 1, kSmallMb16>(rb, re, a, val, op, s, done);
   return launch_wrows<VT, Op, 1, 1, kSmallMb32>(rb, re, a, val, op, s, done);
@@ -701,10 +710,17 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
     }
     if (done) return LGX_OK;
   }
-  // rows of at most 8 entries (7-point operators) at 256^3: FP64 product 350
-  // -> 274, float 295 -> 245 us
-  if (Rounds<Op>::value && TuneClass<Op>::value == 0 && cfg == 3 && a.max_row <= 8) {
-    LGX_CHECK((launch_wrows<VT, Op, 4, 1, kShortMb>(rb, re, a, val, op, s, &done)));
+  // Products of rows of at most 8 entries (7-point operators) without branches, in
+  // six CTAs per SM.  FP64 beyond the 20 tiles per SM that five CTAs hold at once:
+  // 127k rows 4.4 -> 3.6 us, 512k 10.6 -> 10.0, 256^3 350 -> 274, but 69k 2.7 -> 3.2;
+  // float where the matrix streams from memory: 1.7M rows 31.5 -> 26.9, 256^3 295 ->
+  // 245, but 512k 6.9 -> 7.6; float values with FP64 vectors never (bound by their
+  // conversions: 91k 4.1 -> 5.8, 2.7M 87 -> 92).
+  if constexpr (Rounds<Op>::value && TuneClass<Op>::value == 0 &&
+                sizeof(VT) == sizeof(typename Op::X)) {
+    const int64_t tiles = sizeof(VT) == 8 ? 20 : 256;
+    if (cfg == 3 && a.max_row <= 8 && re - rb > (int64_t)sm_count() * tiles * kWarpTileRows)
+      LGX_CHECK((launch_wrows<VT, Op, 4, 1, kShortMb>(rb, re, a, val, op, s, &done)));
     if (done) return LGX_OK;
   }
   // Larger colours of natural-order levels with long rows (over 16 entries on

@@ -32,3 +32,28 @@ def test_jacobi_in_four_warps(cuda, records, points, dims):  # noqa: F811
     m = _matrix(cuda, points, dims)
     x = np.ones(m.row_num())
     assert _shapes(lambda: cuda.jacobi_sweep(m, x, x), "JacobiOp") == [(4, 1, 0)]
+
+
+SMALL8, SMALL32, FOUR, SHORT = (1, 1, 20), (1, 1, 10), (4, 1, 0), (4, 1, 6)
+
+
+# rows on both sides of 2, 8, 20 and 256 tiles per SM
+@pytest.mark.parametrize("kind,points,dims,shape", [
+    ("f64", 7, (8, 16, 304), SMALL8), ("f64", 7, (8, 17, 304), FOUR),
+    ("f64", 7, (20, 16, 304), FOUR), ("f64", 7, (20, 17, 304), SHORT),
+    ("f64", 27, (8, 16, 304), SMALL32), ("f64", 27, (8, 17, 304), FOUR),
+    ("f32", 7, (2, 16, 304), SMALL8), ("f32", 7, (3, 16, 304), FOUR),
+    ("f32", 7, (256, 16, 304), FOUR), ("f32", 7, (256, 17, 304), SHORT),
+    ("f32", 27, (8, 16, 304), SMALL32), ("f32", 27, (8, 17, 304), FOUR),
+    ("mixed", 7, (8, 16, 304), SMALL8), ("mixed", 7, (8, 17, 304), FOUR),
+    ("mixed", 7, (256, 17, 304), FOUR)])
+def test_product_shapes(cuda, records, kind, points, dims, shape):  # noqa: F811
+    import torch
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the lines are in tiles per SM")
+    m = _matrix(cuda, points, dims, 0 if kind == "f64" else 1)
+    x = torch.ones(m.row_num(), dtype=torch.float32 if kind == "f32" else torch.float64,
+                   device="cuda")
+    run = (lambda: cuda.spmv_f32(m, x)) if kind == "f32" else (lambda: cuda.spmv(m, x))
+    assert _shapes(run, "SpmvOp") == [shape]
