@@ -202,6 +202,7 @@ __device__ __forceinline__ double run_row(const Op &op, int64_t r, int32_t i, co
 //   static constexpr bool kList;  const int32_t *rows;  (kList: matrix row r is
 //     vector row rows[r], r itself when rows is null; row() takes both)
 //   static constexpr bool kRounds;  (false: the row walks its entries one by one)
+//   static constexpr bool kBranchForm;  (a sweep whose rows have both forms)
 //   static constexpr bool kReduce;  __device__ void finish(double total) const;
 //   double *partials; unsigned *counter;  (when kReduce)
 template <typename VT, class Op, int KIND>
@@ -285,14 +286,13 @@ __global__ void __launch_bounds__(kTileRows, RowCfg<VT, KIND>::ctas_per_sm)
       if (row < cur.r1) {
         const Stage<VT> sg = stage(s);
         const int64_t b = sg.rp[row - p0], e = sg.rp[row + 1 - p0];
-        contrib += run_row<RowCfg<VT, KIND>::gather, false>(op, row, list_row(op, row, true),
-                                                            sg.col + (b - c0), sg.val + (b - v0),
-                                                            (int)(e - b));
+        contrib += run_row<RowCfg<VT, KIND>::gather, TuneClass<Op>::value == 1>(
+          op, row, list_row(op, row, true), sg.col + (b - c0), sg.val + (b - v0), (int)(e - b));
       }
     } else if (row < cur.r1) {
       const int64_t b = rowptr[row], e = rowptr[row + 1];
-      contrib += run_row<RowCfg<VT, KIND>::gather, false>(op, row, list_row(op, row, true),
-                                                          col + b, val + b, (int)(e - b));
+      contrib += run_row<RowCfg<VT, KIND>::gather, TuneClass<Op>::value == 1>(
+        op, row, list_row(op, row, true), col + b, val + b, (int)(e - b));
     }
     __syncthreads();
     if (NST == 1 && threadIdx.x == 0 && t + G < ntiles) {
@@ -365,6 +365,8 @@ __host__ __device__ constexpr size_t wsmem_bytes(int wpc, int nst, int capw, siz
 constexpr int kSmallMb32 = 10, kSmallMb16 = 14, kSmallMb8 = 20;
 // four-warp CTAs per SM of products whose rows have at most 8 entries
 constexpr int kShortMb = 6;
+// sweeps with a branch per entry in four-warp CTAs, five per SM (launch_rows)
+constexpr int kBranchMb = 5;
 // one-warp CTAs whose lanes gather a tile's entries in storage order into
 // shared memory, before each lane runs its row (launch_spread)
 constexpr int kSpreadMb = 16;
@@ -409,7 +411,8 @@ __global__ void __launch_bounds__(WPC * 32, WrowsBounds<WPC, typename Op::X, MB>
           const int32_t *__restrict__ col, const VT *__restrict__ val, Op op, int *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int W = WrowsBounds<WPC, typename Op::X, MB>::gather;
-  constexpr bool FLAT = WrowsBounds<WPC, typename Op::X, MB>::flat;
+  constexpr bool FLAT = TuneClass<Op>::value == 1 ? MB != kBranchMb
+                                                  : WrowsBounds<WPC, typename Op::X, MB>::flat;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t sb = wstage_bytes(capw, sizeof(VT));
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw) + warp * S;
@@ -634,6 +637,16 @@ inline lgx_status launch_rows_cfg(int64_t rb, int64_t re, int64_t max_row, const
   return LGX_OK;
 }
 
+// sweeps that have their rows with a branch per entry too (FLAT false)
+template <class Op, class = void>
+struct BranchForm {
+  static constexpr bool value = false;
+};
+template <class Op>
+struct BranchForm<Op, std::enable_if_t<Op::kBranchForm>> {
+  static constexpr bool value = true;
+};
+
 // Launches of few tiles (the colours of small levels) in one-warp CTAs: the
 // warps spread evenly over the SMs, and with the rows' whole length in one or
 // two rounds of gathers the launch is one gather latency long.  Up to eight
@@ -643,12 +656,17 @@ inline lgx_status launch_rows_cfg(int64_t rb, int64_t re, int64_t max_row, const
 // 10.7 / 9.6 (float 3.3 / 2.8, 4.3 / 3.7, 4.9 / 4.3), 55k 12.0 / 12.6 (float
 // 5.3 / 5.6); 7-point float 5.5k rows 2.0 / 1.8 us, 37k 2.4 / 2.2, 167k 5.2 /
 // 5.2.  Float products of short rows only up to two tiles per SM (7 points, 7.2k
-// rows 1.54 / 1.45 us, 13.8k 1.49 / 1.54, 32.7k 1.63 / 1.85).
+// rows 1.54 / 1.45 us, 13.8k 1.49 / 1.54, 32.7k 1.63 / 1.85), FP64 sweeps of short
+// rows in colour order up to six (7 points, a sweep of 91k rows, whose largest colour
+// is at 5.6, 20.7 / 17.3 us, of 127k, at 7.8, 19.9 / 22.1).
 template <typename VT, class Op>
 inline lgx_status launch_small(int64_t rb, int64_t re, const Csr &a, const VT *val, const Op &op,
                                cudaStream_t s, bool *done) {
   const bool short_rows = a.max_row <= 8, flt = sizeof(typename Op::X) == 4;
-  const int64_t most = TuneClass<Op>::value == 0 && short_rows && flt ? 2 : 8;
+  int64_t most = 8;
+  if (TuneClass<Op>::value == 0 && short_rows && flt) most = 2;
+  if constexpr (BranchForm<Op>::value)
+    if (short_rows && !flt && !op.rows) most = 6;
   if (re - rb > (int64_t)sm_count() * most * kWarpTileRows) return LGX_OK;
   if (short_rows) return launch_wrows<VT, Op, 1, 1, kSmallMb8>(rb, re, a, val, op, s, done);
   if (a.max_row <= 16)
@@ -721,6 +739,19 @@ inline lgx_status launch_rows(int64_t rb, int64_t re, const Csr &a, const VT *va
     const int64_t tiles = sizeof(VT) == 8 ? 20 : 256;
     if (cfg == 3 && a.max_row <= 8 && re - rb > (int64_t)sm_count() * tiles * kWarpTileRows)
       LGX_CHECK((launch_wrows<VT, Op, 4, 1, kShortMb>(rb, re, a, val, op, s, &done)));
+    if (done) return LGX_OK;
+  }
+  // Colours in colour order that five four-warp CTAs per SM hold at once (20 tiles
+  // per SM), of short or float rows, with a branch per entry: nothing queues behind
+  // their gathers, and the tests of the branch-free rounds cost more than they hide.
+  // Sweeps, branch-free / branches: 7 points FP64 127k rows 22.8 / 19.9 us, 253k 23.4
+  // / 21.2 (373k, largest colour at 23 tiles per SM, 24.7 / 25.7), float 253k 15.6 /
+  // 14.1; 27 points float 512k 102 / 95, 970k (20 tiles) 110 / 100, 2.7M 205 / 228;
+  // FP64 of 27 points always branch-free (512k 151 / 193).
+  if constexpr (BranchForm<Op>::value) {
+    if (cfg == 3 && !op.rows && (sizeof(typename Op::X) == 4 || a.max_row <= 8) &&
+        re - rb <= (int64_t)sm_count() * 20 * kWarpTileRows)
+      LGX_CHECK((launch_wrows<VT, Op, 4, 1, kBranchMb>(rb, re, a, val, op, s, &done)));
     if (done) return LGX_OK;
   }
   // Larger colours of natural-order levels with long rows (over 16 entries on

@@ -706,6 +706,7 @@ struct SorOp {
   using X = XT;
   static constexpr bool kReduce = false;
   static constexpr bool kList = true;
+  static constexpr bool kBranchForm = !kIsBf16<VT>;
   static constexpr int kTuneClass = 1;
   double *partials = nullptr;
   unsigned *counter = nullptr;
@@ -724,9 +725,18 @@ struct SorOp {
       const int m = len - k;
       int32_t cc[W];
       XT xv[W];
-      row_columns<W>(c, k, len, cc);
+      if constexpr (FLAT) {
+        row_columns<W>(c, k, len, cc);
 #pragma unroll
-      for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], u < m && cc[u] != i && cc[u] < end);
+        for (int u = 0; u < W; ++u) ld_if(xv[u], x + cc[u], u < m && cc[u] != i && cc[u] < end);
+      } else {
+#pragma unroll
+        for (int u = 0; u < W; ++u)
+          if (u < m) {
+            cc[u] = c[k + u];
+            xv[u] = cc[u] < end ? x[cc[u]] : XT(0);
+          }
+      }
 #pragma unroll
       for (int u = 0; u < W; ++u) {
         if (u < m) {

@@ -57,3 +57,28 @@ def test_product_shapes(cuda, records, kind, points, dims, shape):  # noqa: F811
                    device="cuda")
     run = (lambda: cuda.spmv_f32(m, x)) if kind == "f32" else (lambda: cuda.spmv(m, x))
     assert _shapes(run, "SpmvOp") == [shape]
+
+
+BRANCH = (4, 1, 5)
+
+
+# rows per colour on both sides of 6, 8 and 20 tiles per SM
+@pytest.mark.parametrize("dtype,points,dims,shape", [
+    ("float64", 7, (12, 16, 304), SMALL8), ("float64", 7, (12, 17, 304), BRANCH),
+    ("float64", 7, (40, 16, 304), BRANCH), ("float64", 7, (40, 17, 304), FOUR),
+    ("float32", 7, (16, 16, 304), SMALL8), ("float32", 7, (16, 17, 304), BRANCH),
+    ("float32", 7, (40, 16, 304), BRANCH), ("float32", 7, (40, 17, 304), FOUR),
+    ("float64", 27, (64, 16, 304), SMALL32), ("float64", 27, (64, 18, 304), FOUR),
+    ("float32", 27, (64, 16, 304), SMALL32), ("float32", 27, (64, 18, 304), BRANCH),
+    ("float32", 27, (160, 16, 304), BRANCH), ("float32", 27, (160, 18, 304), FOUR)])
+def test_sweep_shapes(cuda, records, dtype, points, dims, shape):  # noqa: F811
+    import torch
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the lines are in tiles per SM")
+    i, j, k = np.meshgrid(*[np.arange(d) for d in dims], indexing="ij")
+    c = (i % 2) * 4 + (j % 2) * 2 + k % 2 if points == 27 else (i + j + k) % 2
+    m = _matrix(cuda, points, dims)
+    col = cuda.Colouring.from_array(m, c.ravel().astype(np.int32), 8 if points == 27 else 2)
+    x = torch.ones(m.row_num(), dtype=getattr(torch, dtype), device="cuda")
+    assert _shapes(lambda: cuda.sor_sweep_permuted(col, x, x.clone()), "SorOp") == [shape]
