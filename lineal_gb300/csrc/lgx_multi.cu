@@ -102,10 +102,21 @@ inline unsigned m_ctas(int64_t rows, int G) {
 //    as 0); M_LO: such a sweep on a natural-order level's earlier-colour
 //    halves, the diagonals in pdiag.
 // Matrix row r is vector row rows[r] (natural-order levels), or r itself.  The
-// entries go in chunks of G, a lane loading one, and in batches of four gathers.
+// entries go in chunks of G, a lane loading one, and in batches of B <= G gathers.
+//
+// Launches of so few rows that a column per lane, at least eight lanes (so entries
+// of a chunk) and eight gathers at once take no more than a quarter of the chip last
+// as long as one row's chain, which is shorter so.  Blocked FP64 solves of 7 points,
+// vectors per lane throughout / so, and a warp per row before either, ms: 336 rows, 32
+// columns 2.60 / 2.24 / 2.42, 27 rows, 8 columns 0.78 / 0.70 / 0.71.  With the line at
+// 320000 lanes 64000 rows of 27 points and 32 columns take 25.2 instead of 24.2, and
+// with it at 80000 columns 64000 rows of 7 points and one column 10.63 instead of
+// 10.44.
+constexpr int64_t kMFewLanes = 80000;
+constexpr int kMFewBatch = 8;
 enum MRowMode { M_MUL, M_SOR, M_LO };
 
-template <typename VT, typename XT, int MODE, int V>
+template <typename VT, typename XT, int MODE, int V, int B>
 __global__ void __launch_bounds__(kMThreads)
   k_mrows(int64_t rb, int64_t re, const int64_t *__restrict__ rowptr,
           const int32_t *__restrict__ col, const VT *__restrict__ val,
@@ -113,7 +124,6 @@ __global__ void __launch_bounds__(kMThreads)
           const XT *__restrict__ b, const XT *x, XT *y, XT relax, XT m1, int neg, int ultra,
           int from_zero, int64_t visit_end) {
   constexpr unsigned kAll = 0xffffffffu;
-  constexpr int B = sizeof(XT) == 8 ? 2 : 4;
   const MLane<V> L(G);
   const int64_t r = rb + L.r;
   const bool in = r < re, on = in && L.k0 < K;
@@ -447,12 +457,19 @@ static lgx_status m_rows(int64_t rb, int64_t re, const Csr &p, const VT *val, co
                          const double *pdiag, int K, const XT *b, const XT *x, XT *y, XT relax,
                          int neg, int ultra, int from_zero, cudaStream_t s) {
   if (re <= rb) return LGX_OK;
-  return m_with_vec<XT>(K, [&](auto v, int G) -> lgx_status {
-    k_mrows<VT, XT, MODE, v><<<m_ctas(re - rb, G), kMThreads, 0, s>>>(
+  auto launch = [&](auto v, auto batch, int G) -> lgx_status {
+    k_mrows<VT, XT, MODE, v, batch><<<m_ctas(re - rb, G), kMThreads, 0, s>>>(
       rb, re, p.rowptr.p, p.col.p, val, rows, pdiag, K, G, b, x, y, relax, XT(1) - relax, neg,
       ultra, from_zero, rb);
     LGX_LAUNCH_CHECK();
     return LGX_OK;
+  };
+  const int few = std::max(kMFewBatch, m_group(K, 1));
+  if ((re - rb) * few <= kMFewLanes)
+    return launch(std::integral_constant<int, 1>{}, std::integral_constant<int, kMFewBatch>{},
+                  few);
+  return m_with_vec<XT>(K, [&](auto v, int G) {
+    return launch(v, std::integral_constant<int, sizeof(XT) == 8 ? 2 : 4>{}, G);
   });
 }
 
@@ -586,13 +603,13 @@ struct MState {
 };
 
 // The k_mdot block partials (`which` 0: u.v, 1: w.w) of column k in lane k of
-// warp 0: 32 warps sum strided shares, warp 0 adds them in warp order.  All
-// 1024 threads call it.  (One thread per column summing 1024 partials in turn
-// took 95 us, and 186 for both; now 15 and 27 cold.)
-constexpr int kMScalarThreads = 1024;
+// warp 0: up to 32 warps (as many as partials, m_scalar_threads) sum strided shares,
+// warp 0 adds them in warp order.  All threads call it.  (One thread per column
+// summing 1024 partials in turn took 95 us, and 186 for both; now 15 and 27 cold.)
+inline unsigned m_scalar_threads(unsigned g) { return 32 * std::min(g, 32u); }
 __device__ double m_column_sum(const double *partials, unsigned g, int which) {
   __shared__ double sh[32][kMaxRhs];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
   double a = 0.0;
 #pragma unroll 4
   for (unsigned q = w; q < g; q += 32) a += partials[((size_t)q * 2 + which) * kMaxRhs + lane];
@@ -601,7 +618,7 @@ __device__ double m_column_sum(const double *partials, unsigned g, int which) {
   __syncthreads();
   double t = 0.0;
   if (w == 0)
-    for (int v = 0; v < 32; ++v) t += sh[v][lane];
+    for (int v = 0; v < warps; ++v) t += sh[v][lane];
   return t;
 }
 
@@ -790,7 +807,7 @@ static lgx_status pcg_multi(const lgx_matrix *a, lgx_amg &h, int K, const double
     LGX_CHECK(apply(nullptr, P.p, Q.p));
     k_mdot<double, false><<<gdot, kMThreads, 0, s>>>(n, K, P.p, Q.p, partials.p);
     LGX_LAUNCH_CHECK();
-    k_malpha<<<1, kMScalarThreads, 0, s>>>(gdot, K, partials.p, state.p, alpha_d.p);
+    k_malpha<<<1, m_scalar_threads(gdot), 0, s>>>(gdot, K, partials.p, state.p, alpha_d.p);
     k_mupdate<<<egrid(nk), 256, 0, s>>>(n, K, alpha_d.p, P.p, Q.p, X.p, R.p, rere ? nullptr : rf);
     LGX_LAUNCH_CHECK();
     if (rere) {
@@ -800,7 +817,7 @@ static lgx_status pcg_multi(const lgx_matrix *a, lgx_amg &h, int K, const double
     // Z = M R ; beta = R.Z / rho ; P = Z + beta P
     LGX_CHECK(precondition());
     LGX_CHECK(dots_rz());
-    k_mbeta<<<1, kMScalarThreads, 0, s>>>(gdot, K, partials.p, rtol, state.p, beta_d.p);
+    k_mbeta<<<1, m_scalar_threads(gdot), 0, s>>>(gdot, K, partials.p, rtol, state.p, beta_d.p);
     k_mxpby<XT><<<egrid(nk), 256, 0, s>>>(n, K, beta_d.p, z, P.p);
     LGX_LAUNCH_CHECK();
     return LGX_OK;
@@ -836,7 +853,7 @@ static lgx_status pcg_multi(const lgx_matrix *a, lgx_amg &h, int K, const double
   LGX_CHECK(to_float());
   LGX_CHECK(precondition());
   LGX_CHECK(dots_rz());
-  k_minit<<<1, kMScalarThreads, 0, s>>>(gdot, K, partials.p, maxit, state.p);
+  k_minit<<<1, m_scalar_threads(gdot), 0, s>>>(gdot, K, partials.p, maxit, state.p);
   LGX_LAUNCH_CHECK();
   if constexpr (kFloat) {
     k_mconvert<float, double><<<egrid(nk), 256, 0, s>>>(nk, z, P.p);
