@@ -590,7 +590,14 @@ lgx_status solo_solve(bool cg, const lgx_matrix *a, const double *d_b, double *d
   A.err = device_error_flag();
   A.out = out.p;
   void *args[] = {&A};
-  LGX_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kST), args, 0, s));
+  const cudaError_t launched = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kST), args, 0, s);
+  if (launched == cudaErrorCooperativeLaunchTooLarge) {
+    // less of the device than its properties say (a shared or divided one): the
+    // launches take the solve, x is as it was
+    cudaGetLastError();
+    return LGX_OK;
+  }
+  LGX_CUDA(launched);
   count_launch();
   SoloResult h{};
   LGX_CUDA(cudaMemcpyAsync(&h, out.p, sizeof(h), cudaMemcpyDeviceToHost, s));
