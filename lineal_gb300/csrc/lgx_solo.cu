@@ -83,9 +83,12 @@ struct SoloShared {
 // Up to kSoloMaxRows entries below 2^501 have a finite sum of squares.  BiCGStab
 // takes the norm of its half residual only where there are larger ones (for its
 // error on overflow); that there are travels as the top bit of the barriers'
-// counter, which counts to less than 2^31 (at most a million iterations).
+// counter, which counts to less than 2^31: at most seven barriers an iteration, of
+// kSoloMaxCtas CTAs, in kSoloMaxIterations (beyond them, the launches).
 constexpr int kSoloHuge = 1023 + 501;
 constexpr unsigned kSoloHugeBit = 0x80000000u;
+constexpr int64_t kSoloMaxIterations = 900000;
+static_assert(7 * (kSoloMaxIterations + 1) * kSoloMaxCtas < (int64_t)kSoloHugeBit, "counter");
 
 __device__ __forceinline__ bool finite_bits(double v) { return exponent_field(v) != 0x7ff; }
 
@@ -532,8 +535,8 @@ lgx_status solo_solve(bool cg, const lgx_matrix *a, const double *d_b, double *d
   *done = false;
   const int64_t n = a->n;
   if ((p->precon != LGX_PRECON_NONE && p->precon != LGX_PRECON_JACOBI) || !p->use_graphs ||
-      (cg && p->flexible && p->precon != LGX_PRECON_NONE) || n < 1 || n > kSoloMaxRows || p->maxit < 0 || p->maxit > 1000000 ||
-      overlap(d_b, d_x, sizeof(double) * (size_t)n))
+      (cg && p->flexible && p->precon != LGX_PRECON_NONE) || n < 1 || n > kSoloMaxRows ||
+      p->maxit < 0 || p->maxit > kSoloMaxIterations || overlap(d_b, d_x, sizeof(double) * (size_t)n))
     return LGX_OK;
   int dev = 0, coop = 0;
   LGX_CUDA(cudaGetDevice(&dev));
