@@ -428,7 +428,9 @@ typedef struct lgx_amg lgx_amg;
  * (IndependentAggregationSink + BaseAggregator), Galerkin coarse matrices
  * (coarsen_matrix), multicolour SOR smoothers and a dense FP64 coarsest
  * solver.  finest_colouring may be NULL (JP colouring is computed).  The
- * finest matrix must stay alive while the hierarchy is used.  Synchronises
+ * finest matrix must stay alive while the hierarchy is used.  Levels hold
+ * their entries twice where that takes at most a third of the free device
+ * memory, else once (the same V-cycle, bit for bit).  Synchronises
  * `stream` (level sizes decide the loop). */
 lgx_status lgx_amg_setup(const lgx_matrix *a, const lgx_amg_params *p,
                          const lgx_colouring *finest_colouring, lgx_stream stream,
@@ -524,12 +526,14 @@ lgx_status lgx_direct_solve(const lgx_direct *d, const double *d_b, double *d_x,
 lgx_status lgx_direct_destroy(lgx_direct *d);
 
 /* One V-cycle from a zero initial guess: x = M^-1 b (MultiGridSolver::
- * Instance::apply, multigrid/solver.hpp:41-176, REGULAR cycle, 1 iteration). */
+ * Instance::apply, multigrid/solver.hpp:41-176, REGULAR cycle, 1 iteration).
+ * d_x may overlap d_b. */
 lgx_status lgx_amg_vcycle(lgx_amg *h, const double *d_b, double *d_x, lgx_stream stream);
 /* Autotunes (see lgx_matrix_autotune) every smoothed level of a hierarchy:
  * its residual and its forward SOR sweep in the value and vector types its
  * cycles read, and with cycle_f32 also the finest level's FP64 product (the
- * outer Krylov SpMV).  A level keeps its fastest shapes only if a whole
+ * outer Krylov SpMV; the choice is this hierarchy's, not the matrix's).  A
+ * level keeps its fastest shapes only if a whole
  * V-cycle (graph replays, timed) is also faster with them than with the
  * process-wide configuration there; otherwise `config` reports the
  * process-wide one.  Writes up to max_out entries to *out and the number
@@ -665,9 +669,9 @@ lgx_status lgx_krylov_destroy(lgx_krylov *k);
  * -(1 + max(+-v_d, 0)) toward each neighbour and the sum of the six
  * magnitudes on the diagonal) solved by Jacobi-preconditioned BiCGStab
  * (bicgstab/solver.hpp:73-151, Jacobi from zero with `relax`) in one
- * persistent launch: each CTA solves whole systems taken from a work queue,
- * largest first, with the termination rule of run_iterative_solver
- * (runner.hpp:17-84) evaluated on the device.  No reference counterpart for
+ * persistent launch: clusters of CTAs solve the larger systems, single CTAs the
+ * others, taken from work queues, largest first, with the termination rule of
+ * run_iterative_solver (runner.hpp:17-84) evaluated on the device.  No reference counterpart for
  * the batching itself.
  * ---------------------------------------------------------------------- */
 typedef struct {
