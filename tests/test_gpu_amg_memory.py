@@ -16,14 +16,14 @@ def _free():
     return torch.cuda.mem_get_info()[0]
 
 
-@pytest.mark.parametrize("form", ["fp64", "coarse_f32"])
+@pytest.mark.parametrize("form", ["fp64", "coarse_f32", "f32"])
 def test_setup_with_little_memory(cuda, form):
     import torch
 
     dims = (100, 100, 100)
     n = int(np.prod(dims))
     m = cuda.gen_27pt(dims, np.exp(np.random.default_rng(3).standard_normal(n)))
-    kw = dict(coarse_f32=form == "coarse_f32")
+    kw = dict(coarse_f32=form == "coarse_f32", cycle_f32=form == "f32")
     b = torch.from_numpy(np.random.default_rng(4).uniform(-1, 1, n)).cuda()
     out = torch.empty_like(b)
     want = cuda.HierarchyWright(**kw).instantiate(m).vcycle(b).clone()
@@ -33,7 +33,8 @@ def test_setup_with_little_memory(cuda, form):
     try:
         h = cuda.HierarchyWright(**kw).instantiate(m)
         h.vcycle(b, out=out)
-        res = cuda.pcg(m, b, precon=cuda.PRECON_AMG, amg=h, rtol=1e-6, maxit=100)
+        res = cuda.pcg(m, b, precon=cuda.PRECON_AMG, amg=h, rtol=1e-6, maxit=100,
+                       flexible=form == "f32")
     finally:
         del ballast
         torch.cuda.empty_cache()
